@@ -177,18 +177,29 @@ struct SellMat {
     int64_t nns() const { return (int64_t)nslices * 32 * nd; }
 };
 
-// Incomplete-Cholesky factor of the IML solver's IC preconditioner (icprec.cu):
-// forward rows (entries of the transposed columns), backward rows (each row's
-// own column below the diagonal), the diagonal, and both level schedules.
+// Dataflow schedule of one triangular solve (icprec.cu): the structure it was made
+// for, the units in order, and where the factor's entries go.
+struct FlowSched {
+    int n = 0;
+    std::vector<int64_t> ptr;      // rows of the triangle the schedule belongs to
+    std::vector<int> col;
+    std::vector<int> unit;         // 4 per unit: first row, rows, slots per lane, first slot
+    std::vector<int> csrc;         // 16 per unit: entry of (row, earlier row of the unit), -1 none
+    std::vector<int> slot_col, slot_src;   // column and entry of every lane slot, -1 none
+    bool uploaded = false;
+    DBuf<int> d_unit, d_col;
+    DBuf<double> d_coef, d_val;
+};
+
+// Incomplete-Cholesky (or ILU) factor of the IML solver's preconditioners (icprec.cu).
 struct IcFactor {
     int64_t version = -1;
     int kind = 0;   // 4 incomplete Cholesky, 2 ILU (lsprecond)
     int n = 0;
-    DBuf<int64_t> fptr, bptr;
-    DBuf<int> fcol, bcol, frows, brows;
-    DBuf<double> fval, bval, diag, work;
-    std::vector<int> flev, blev;   // level starts into frows / brows
-    DBuf<int> d_flev, d_blev;      // the same on the device
+    FlowSched fwd, bwd;
+    DBuf<double> work;
+    int cluster = 0;              // CTAs of the solve's cluster (0 = not looked up)
+    bool cluster_local = false;   // ... for the shared-memory form
 };
 
 // LDL^T factor of the direct solver (direct.cu): dense band of n x (bw+1)
@@ -375,9 +386,9 @@ int build_sell(ogb_model *md, ogb_mtrx *m);
 // values into it.
 int build_half(ogb_ctx *ctx, SellMat &S);
 // icprec.cu: the IC factor of m (host, cached per matrix version) and z = M^-1 r
-// (device, level-scheduled; kernels skip once sc reports done).
+// with r.z -> rho and beta (device; skipped once sc reports done).
 int build_ic(ogb_mtrx *m);
-int launch_ic_solve(ogb_mtrx *m, const double *r, double *z, const PcgScal *sc);
+int launch_ic_solve(ogb_mtrx *m, const double *r, double *z, PcgScal *sc);
 int refresh_half(ogb_ctx *ctx, SellMat &S);
 
 // element.cu

@@ -359,6 +359,39 @@ def test_iml_preconditioners_many_levels(pc, native_lib, oracle):
     assert rel(u, ref["u"]) < 1e-9
 
 
+@pytest.mark.parametrize("mesh,size,pc", [("hex", (1, 1, 1), 4), ("hex", (2, 1, 1), 2), ("quad", 5, 4), ("quad", 13, 2),
+                                          ("tet", 5, 4), ("hex", (33, 7, 6), 2), ("hex", (60, 12, 12), 4)])
+def test_iml_triangular_solves_sizes(mesh, size, pc, native_lib, oracle):
+    """The dataflow triangular solves at their edges: one unit of rows, units of
+    two DOFs per node, more units than warps, and a vector above the
+    shared-memory copies' 28,800 rows (60 x 12 x 12: 30,720), against the oracle's
+    IML CG (the largest: the diagonal-preconditioned solve) to the same tolerance. Two CG solutions at a relative residual of 1e-12
+    are within the preconditioned condition number (below 1e4 here) of it."""
+    from oofem_gb300 import meshgen as mg
+    if mesh == "hex":
+        m = mg.hex_cantilever(*size, jitter=0.2, seed=5)
+    elif mesh == "quad":
+        m = mg.quad_rve(size, seed=5)
+    else:
+        m = mg.tet_cube_linear(size, jitter=0.15, seed=5)
+    model = native_lib.GpuModel(native_lib.Context(0), m)
+    A = native_lib.GpuCsrMtrx(model.ctx)
+    A.set_preconditioner(pc)
+    u, _, info = model.linear_static(A, rtol=1e-12)
+    assert info.status == 0
+    if m.nnodes < 5000:
+        ref = oracle.linear_static(oracle.mesh_dict(m), rtol=1e-12, precond=pc)["u"]
+    else:
+        B = native_lib.GpuCsrMtrx(model.ctx)
+        model.build_matrix(B)
+        ref, _, _ = model.linear_static(B, rtol=1e-12, maxit=100000)
+        model.build_matrix(A)
+    assert rel(u, ref) < 1e-8, rel(u, ref)
+    # bitwise reproducible
+    u2, _, i2 = model.linear_static(A, rtol=1e-12)
+    assert np.array_equal(u, u2) and info.iterations == i2.iterations
+
+
 @pytest.mark.parametrize("kind", ["hex", "quad", "tet"])
 def test_block_jacobi_mixed_solve(kind, native_lib, oracle):
     """Mixed solves preconditioned by the FP32 inverses of the node diagonal
