@@ -11,19 +11,31 @@
 // pivoting stays inside each column's profile, which for the full symmetric
 // pattern is bounded by the half bandwidth bw = max_i (last column of row i - i).
 //
-// What is GB300-native: the factor lives in a dense band of n x (bw+1) doubles
-// in HBM, column-major (column j holds L(j..j+bw, j), its diagonal slot holds
-// d_j), and is computed right-looking in panels of 32 columns -- one CTA
-// factors the panel's 32 x 32 diagonal block in shared memory, one thread per
-// row below it solves that row against the block (L21 = A21 L11^-T D^-1), then
-// a 2-D grid of 32 x 32 tiles applies the panel's rank-32 update to the trailing
-// band (shared-memory staged, FP64 FMAs). The solves run in one
-// CTA in blocks of 32 equations: one warp resolves the 32 x 32 triangle with
-// shuffles, the other warps apply the block to the rows below (forward) or
-// reduce the rows below into the block (backward). Every sum has a fixed order,
-// so results are bitwise reproducible. The summation order differs from the
-// reference's column-by-column Crout loop, so factors agree to rounding.
+// What is GB300-native: the factor lives in a dense band, column-major (column j
+// holds L(j..j+bw, j), its diagonal slot holds d_j), and is computed right-looking
+// in panels of 32 columns: one CTA factors the panel's 32 x 32 diagonal block and
+// inverts its unit triangle, the rows below are multiplied by that inverse
+// (L21 = A21 L11^-T D^-1), and a 2-D grid of 32 x 32 tiles applies the panel's
+// rank-32 update to the trailing band. Every sum has a fixed order, so results are
+// bitwise reproducible; the order differs from the reference's column-by-column
+// Crout loop, so factors agree to rounding.
+//
+// The equations are reordered first (ldl_order): factoring costs n bw^2, and a
+// mesh numbered along its longest side has several times the half bandwidth of the
+// same mesh numbered across it. The band is then factored from both ends at once:
+// with m >= bw rows set aside in the middle, the n1 rows before them and the n1
+// rows after them do not meet, so their panels run in the same launches as two
+// bands (the second one reversed), halving the chain of panels; the middle rows
+// take both ends' updates and are factored last. A matrix whose reordered
+// elimination meets a zero pivot (an indefinite matrix; there is no pivoting) is
+// factored again in its own order, from one end.
+//
+// Measured (GB300, 60 x 12 x 12 hexes, 30.4 k equations): half bandwidth 2,567 ->
+// 551; factorization 271 -> 19 ms, substitution 62 -> 3.7 ms.
 #include <math.h>
+
+#include <algorithm>
+#include <vector>
 
 #include "internal.cuh"
 #include "reduce.cuh"
@@ -33,8 +45,7 @@ namespace ogb {
 namespace {
 
 constexpr int PANEL = 32;        // columns per panel
-constexpr int PANEL_THREADS = 1024;
-constexpr int SOLVE_THREADS = 1024;   // 32 warps: one per column of a 32-equation block
+constexpr int EXCLUSIVE_SMEM = 120 * 1024;   // more than half an SM's shared memory
 
 inline unsigned nblk(int64_t n) { return (unsigned)ceil_div(n > 0 ? n : 1, NTHREADS); }
 
@@ -49,204 +60,533 @@ __global__ void k_ldl_bandwidth(int n, const int64_t *__restrict__ rowptr, const
     if (span > 0) atomicMax(bw, span);
 }
 
-// Band from the upper triangle of the CSR rows: entry (i, j), j >= i, is
-// L-column i at offset j - i (the lower triangle K(j, i) of a symmetric matrix).
-// One warp per row.
-__global__ void k_ldl_fill(int n, int bw, const int64_t *__restrict__ rowptr, const int *__restrict__ colind,
-                           const double *__restrict__ val, double *__restrict__ band)
+// The two bands of a factorization (one when `nb` is 1): a[b] has rows N[b], the
+// first `nelim` of which the two bands eliminate in the same launches; xinv[b]
+// holds the 32 x 32 inverse of every panel's unit triangle.
+struct Bands {
+    double *a[2], *xinv[2];
+    int N[2];
+    int bw;
+};
+
+// Band entries from the upper triangle of the CSR rows (the lower triangle of a
+// symmetric matrix): K(i, j), j >= i, goes to the position (r, c), r > c, that the
+// order gives it; rows from mid on that do not meet the first band's columns belong
+// to the second band, reversed. One warp per row.
+__global__ void k_ldl_fill(int n, int mid, const int64_t *__restrict__ rowptr, const int *__restrict__ colind,
+                           const double *__restrict__ val, const int *__restrict__ pos, Bands B)
 {
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (w >= n) return;
     const int i = (int)w;
-    const int64_t ld = (int64_t)bw + 1;
+    const int64_t ld = (int64_t)B.bw + 1;
+    const int pi = pos ? pos[i] : i;
     for (int64_t k = rowptr[i] + lane; k < rowptr[i + 1]; k += 32) {
         const int j = colind[k];
-        if (j >= i && j < n) band[(int64_t)i * ld + (j - i)] = val[k];
+        if (j < i || j >= n) continue;
+        const int pj = pos ? pos[j] : j;
+        const int r = max(pi, pj), c = min(pi, pj);
+        if (r < mid) B.a[0][(int64_t)c * ld + (r - c)] = val[k];
+        else B.a[1][(int64_t)(n - 1 - r) * ld + (r - c)] = val[k];
     }
 }
 
-// Diagonal block of panel [k0, k1) (P = k1 - k0 <= 32 columns): its lower
-// triangle is loaded into shared memory (thread (r, s) of a 32 x 32 CTA owns
-// entry (r, s)) and factored in place, column by column: d_j = A(j,j), the
-// columns s > j receive A(r, s) -= l_rj A(s, j) (A(s, j) not yet scaled), then
-// column j is scaled to l_rj = A(r, j) / d_j. L11 and D go back to the band. A
-// zero or non-finite pivot sets *status to the 1-based equation and stops this
-// and every later launch.
-__global__ void __launch_bounds__(PANEL_THREADS) k_ldl_diag(int n, int bw, double *__restrict__ band, int k0, int k1,
-                                                            int *status)
+// Diagonal block of panel [k0, k0 + P) of a band (P <= 32): L D L^T and the inverse X
+// of its unit triangle together, as row operations on the full symmetric 32 x 32
+// block E (a warp holds rows warp + 8 q, a lane one column). In step j row j's owner
+// publishes W = E(j, :) / d_j (with 1 / d_j in column j), and every row r > j
+// subtracts E(r, j) W. Right of the diagonal that is the elimination of A, left of
+// it and in column j the same operations build X = L^-1. One barrier per step; the
+// chain is the pivot's reciprocal, which the next row's owner takes right after
+// that row's update, its first of the step: 0.75 us per step, most of it FP64
+// latency. (Three barriers and a division in every row: 52 us per block; this
+// scheme 24.8 us in eight warps and 24.2 us in 32, so the CTA that has updated the
+// block can go on with it.) A zero or
+// non-finite pivot sets *status to the 1-based equation of the band (negative:
+// second band) and stops every later launch.
+constexpr int ROWS_PER_WARP = PANEL / (NTHREADS / 32);
+__device__ __forceinline__ void factor_block(const Bands &B, int band, int k0, int P, double (&e)[ROWS_PER_WARP],
+                                             double (&W)[2][PANEL], int &bad, int *status)
 {
-    if (*status) return;
-    __shared__ double A[PANEL][PANEL + 1];
-    __shared__ double lj[PANEL];
+    const int bw = B.bw, warp = threadIdx.x >> 5, c = threadIdx.x & 31;
+    double *A = B.a[band];
     const int64_t ld = (int64_t)bw + 1;
-    const int P = k1 - k0;
-    const int r = threadIdx.x >> 5, c = threadIdx.x & 31;
-    const bool own = r < P && c <= r && r - c <= bw;
-    A[r][c] = own ? band[(int64_t)(k0 + c) * ld + (r - c)] : 0.0;
+    double l[ROWS_PER_WARP];
+#pragma unroll
+    for (int q = 0; q < ROWS_PER_WARP; ++q) l[q] = 0.0;
+    if (threadIdx.x == 0) bad = 0;
     __syncthreads();
-    for (int j = 0; j < P; ++j) {
-        const double d = A[j][j];
-        if (!(d != 0.0) || !isfinite(d)) {
-            if (threadIdx.x == 0) *status = k0 + j + 1;
-            return;   // every thread read the same d: a uniform exit
+    auto publish = [&](int j, double row) {   // row j's warp
+        const double d = __shfl_sync(0xffffffffu, row, j);
+        if ((!(d != 0.0) || !isfinite(d)) && c == 0) bad = j + 1;
+        const double r = 1.0 / d;
+        W[j & 1][c] = c == j ? r : row * r;
+    };
+    if (warp == 0) publish(0, e[0]);
+#pragma unroll
+    for (int jq = 0; jq < ROWS_PER_WARP; ++jq)
+#pragma unroll 1
+        for (int jw = 0; jw < NTHREADS / 32; ++jw) {
+            const int j = jw + (NTHREADS / 32) * jq;
+            if (j >= P) break;
+            __syncthreads();
+            if (bad) {
+                if (threadIdx.x == 0) atomicCAS(status, 0, band ? -(k0 + bad) : k0 + bad);
+                return;   // every thread read the same flag after the barrier: a uniform exit
+            }
+            const double w = W[j & 1][c];
+#pragma unroll
+            for (int q = jq; q < ROWS_PER_WARP; ++q) {
+                const int r = warp + (NTHREADS / 32) * q;
+                if (r <= j) continue;
+                const double f = __shfl_sync(0xffffffffu, e[q], j);
+                const double t = fma(-f, w, c == j ? 0.0 : e[q]);
+                if (c == j) l[q] = -t;
+                e[q] = t;
+                if (r == j + 1 && r < P) publish(r, t);
+            }
         }
-        if (c == j && r > j && r < P) lj[r] = A[r][j] / d;
-        __syncthreads();
-        if (c > j && r >= c && r < P) A[r][c] -= lj[r] * A[c][j];
-        __syncthreads();
-        if (c == j && r > j && r < P) A[r][j] = lj[r];
-        __syncthreads();
+#pragma unroll
+    for (int q = 0; q < ROWS_PER_WARP; ++q) {
+        const int r = warp + (NTHREADS / 32) * q;
+        if (r < P && c <= r && r - c <= bw) A[(int64_t)(k0 + c) * ld + (r - c)] = c == r ? e[q] : l[q];
+        B.xinv[band][(int64_t)k0 * PANEL + r * PANEL + c] = c < r ? e[q] : c == r ? 1.0 : 0.0;
     }
-    if (own) band[(int64_t)(k0 + c) * ld + (r - c)] = A[r][c];
 }
 
-// Rows below the diagonal block, one thread per row i in [k1, min(n, k1 + bw)):
-// y = a L11^-T by forward substitution over the panel columns in order
-// (y_j = a_j - sum_{p<j} y_p l_jp), then L(i, j) = y_j / d_j. Entries outside
-// the band (i - j > bw) are zero and stay unwritten.
-__global__ void __launch_bounds__(NTHREADS) k_ldl_subpanel(int n, int bw, double *__restrict__ band, int k0, int k1,
-                                                           const int *status)
+// First panel of a range: its diagonal block as it stands in the band.
+__global__ void __launch_bounds__(NTHREADS) k_ldl_diag(Bands B, int k0, int *status)
 {
     if (*status) return;
-    __shared__ double L[PANEL][PANEL + 1];
-    __shared__ double dd[PANEL];
+    __shared__ double W[2][PANEL];
+    __shared__ int bad;
+    const int bw = B.bw, band = blockIdx.x, P = min(PANEL, B.N[band] - k0);
+    const int c = threadIdx.x & 31;
+    double e[ROWS_PER_WARP];
+#pragma unroll
+    for (int q = 0; q < ROWS_PER_WARP; ++q) {
+        const int r = (threadIdx.x >> 5) + (NTHREADS / 32) * q, hi = max(r, c), lo = min(r, c);
+        e[q] = hi < P && hi - lo <= bw ? B.a[band][(int64_t)(k0 + lo) * ((int64_t)bw + 1) + (hi - lo)] : (r == c ? 1.0 : 0.0);
+    }
+    factor_block(B, band, k0, P, e, W, bad, status);
+}
+
+// Rows below the diagonal block, SUB_ROWS per CTA, a warp per row and a lane per
+// panel column: y_c = sum_{p <= c} X(c, p) a_p (the row times L11^-T), L(i, c) =
+// y_c / d_c. Entries outside the band (i - c > bw) are zero and stay unwritten.
+// Eight rows per CTA spread the FP64 work of the few hundred rows of a panel over
+// the SMs (one thread per row and a 32-step substitution on three SMs took 57.7 us).
+constexpr int SUB_ROWS = 8;
+__global__ void __launch_bounds__(NTHREADS) k_ldl_subpanel(Bands B, int k0, const int *status)
+{
+    if (*status) return;
+    __shared__ double X[PANEL][PANEL + 1];
+    const int bw = B.bw, band = blockIdx.y;
+    double *A = B.a[band];
     const int64_t ld = (int64_t)bw + 1;
-    const int P = k1 - k0;
-    for (int t = threadIdx.x; t < PANEL * PANEL; t += blockDim.x) {
-        const int r = t >> 5, c = t & 31;
-        L[r][c] = (r < P && c < r && r - c <= bw) ? band[(int64_t)(k0 + c) * ld + (r - c)] : 0.0;
-        if (r == c) dd[r] = r < P ? band[(int64_t)(k0 + r) * ld] : 1.0;
-    }
+    const int P = min(PANEL, B.N[band] - k0), k1 = k0 + P;
+    const int lane = threadIdx.x & 31, i = k1 + blockIdx.x * SUB_ROWS + (threadIdx.x >> 5);
+    const int e = (int)min((int64_t)B.N[band], (int64_t)k1 + bw);
+    const int off = i - (k0 + lane);
+    const bool on = i < e && lane < P && off <= bw;
+    double *ap = A + (int64_t)(k0 + lane) * ld + off;
+    const double a = on ? *ap : 0.0, d = lane < P ? A[(int64_t)(k0 + lane) * ld] : 1.0;
+    for (int t = threadIdx.x; t < PANEL * PANEL; t += NTHREADS)
+        X[t >> 5][t & 31] = B.xinv[band][(int64_t)k0 * PANEL + t];
     __syncthreads();
-    const int64_t i = (int64_t)k1 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t e = min((int64_t)n, (int64_t)k1 + bw);
-    if (i >= e) return;
-    double y[PANEL];
+    double y = a;
 #pragma unroll
-    for (int j = 0; j < PANEL; ++j) {
-        const int64_t off = i - (k0 + j);
-        y[j] = (j < P && off <= bw) ? band[(int64_t)(k0 + j) * ld + off] : 0.0;
+    for (int p = 0; p < PANEL - 1; ++p) {
+        const double v = __shfl_sync(0xffffffffu, a, p);
+        if (p < lane) y = fma(X[lane][p], v, y);
     }
-#pragma unroll
-    for (int j = 1; j < PANEL; ++j) {
-        double s = y[j];
-#pragma unroll
-        for (int p = 0; p < j; ++p) s -= y[p] * L[j][p];
-        y[j] = s;
-    }
-#pragma unroll
-    for (int j = 0; j < PANEL; ++j) {
-        const int64_t off = i - (k0 + j);
-        if (j < P && off <= bw) band[(int64_t)(k0 + j) * ld + off] = y[j] / dd[j];
-    }
+    if (on) *ap = y / d;
 }
 
 // Trailing update of panel [k0, k1) on the band rows/columns [k1, e),
-// e = min(n, k1 + bw): A(i, c) -= sum_p L(i, p) d_p L(c, p) for c <= i, both
-// within the band of the panel column p. Tile (ti, tc) of 32 x 32, lower tiles
-// only; the panel rows of the tile are staged in shared memory (Li transposed,
+// e = min(N, k1 + bw): A(i, c) -= sum_p L(i, p) d_p L(c, p) for c <= i, both
+// within the band of the panel column p. One CTA per 32 x 32 tile of the lower
+// triangle; the panel rows of the tile are staged in shared memory (Li transposed,
 // so the lanes read consecutive words). Lane a takes row i0 + a, so the lanes of
-// a warp read and write 32 consecutive entries of one band column.
-__global__ void __launch_bounds__(NTHREADS) k_ldl_trailing(int n, int bw, double *__restrict__ band, int k0, int k1,
-                                                           const int *status)
+// a warp read and write 32 consecutive entries of one band column; the four columns
+// of a warp are four independent chains. With `next`, the CTA of tile (0, 0), the
+// next panel's diagonal block, goes on to factor it while the others update theirs.
+// FP64-bound where there are tiles enough: at a half bandwidth of 2,567 it runs at
+// the FP64 rate (105 M multiply-adds in 175 us); at 551 and two bands 342 tiles
+// leave two to three per SM: 32.7 us with the factored block, 44.8 us and
+// 24.4 us as two launches.
+__global__ void __launch_bounds__(NTHREADS) k_ldl_trailing(Bands B, int nb, int k0, int next, int *status)
 {
     if (*status) return;
-    const int ti = blockIdx.y, tc = blockIdx.x;
-    if (ti < tc) return;
+    // both bands' first tiles come first: they factor the next diagonal blocks
+    const int band = blockIdx.x % nb, tile = blockIdx.x / nb, bw = B.bw;
+    // tile of the lower triangle: row ti has ti + 1 tiles
+    int ti = (int)((sqrtf(8.0f * tile + 1.0f) - 1.0f) * 0.5f);
+    while ((ti + 1) * (ti + 2) / 2 <= tile) ++ti;
+    while (ti * (ti + 1) / 2 > tile) --ti;
+    const int tc = tile - ti * (ti + 1) / 2;
     __shared__ double Li[PANEL][32];       // L(i, p) * d_p, [p][a]
     __shared__ double Lc[32][PANEL + 1];   // L(c, p), [b][p]
+    __shared__ double E[PANEL][PANEL + 1]; // the next diagonal block
+    __shared__ double W[2][PANEL];
+    __shared__ int bad;
+    double *A = B.a[band];
     const int64_t ld = (int64_t)bw + 1;
-    const int e = (int)min((int64_t)n, (int64_t)k1 + bw);
+    const int P = min(PANEL, B.N[band] - k0), k1 = k0 + P;
+    const int e = (int)min((int64_t)B.N[band], (int64_t)k1 + bw);
     const int i0 = k1 + 32 * ti, c0 = k1 + 32 * tc;
-    const int P = k1 - k0;
-    for (int t = threadIdx.x; t < 32 * PANEL; t += blockDim.x) {
-        const int p = t / 32, a = t % 32;
-        if (p >= P) {
-            Li[p][a] = 0.0;
-            Lc[a][p] = 0.0;
-            continue;
-        }
-        const int j = k0 + p;
-        const double *cjp = band + (int64_t)j * ld;
-        const int i = i0 + a, c = c0 + a;
-        Li[p][a] = (i < e && i - j <= bw) ? cjp[i - j] * cjp[0] : 0.0;
-        Lc[a][p] = (c < e && c - j <= bw) ? cjp[c - j] : 0.0;
-    }
-    __syncthreads();
+    const bool diag = next && tile == 0;
     const int a = threadIdx.x & 31, b0 = threadIdx.x >> 5;
     const int i = i0 + a;
-    if (i >= e) return;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int b = b0 + 8 * q;
-        const int c = c0 + b;
-        if (c >= e || i < c || i - c > bw) continue;
-        double s = 0.0;
-        for (int p = 0; p < P; ++p) s += Li[p][a] * Lc[b][p];
-        band[(int64_t)c * ld + (i - c)] -= s;
+    for (int q = 0; q < PANEL / (NTHREADS / 32); ++q) {
+        const int p = b0 + q * (NTHREADS / 32), j = k0 + p, c = c0 + a;
+        const double *cjp = A + (int64_t)j * ld;
+        Li[p][a] = (p < P && i < e && i - j <= bw) ? cjp[i - j] * cjp[0] : 0.0;
+        Lc[a][p] = (p < P && c < e && c - j <= bw) ? cjp[c - j] : 0.0;
+    }
+    if (diag) {
+        // lower triangle of the next diagonal block, 528 entries packed over the
+        // threads (half the FP64 work of the tile), handed over through shared memory
+        const int Pn = min(PANEL, B.N[band] - k1);
+        double old[3], sum[3];
+        int rr[3], cc[3];
+#pragma unroll
+        for (int h = 0; h < 3; ++h) {
+            const int t = threadIdx.x + h * NTHREADS;
+            int r = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
+            if ((r + 1) * (r + 2) / 2 <= t) ++r;
+            if (r * (r + 1) / 2 > t) --r;
+            rr[h] = r;
+            cc[h] = t - r * (r + 1) / 2;
+            const bool in = t < PANEL * (PANEL + 1) / 2 && r < Pn && r - cc[h] <= bw;
+            if (!in) rr[h] = -1;
+            old[h] = in ? A[(int64_t)(k1 + cc[h]) * ld + (r - cc[h])] : 0.0;
+            sum[h] = 0.0;
+        }
+        for (int t = threadIdx.x; t < PANEL * PANEL; t += NTHREADS) E[t >> 5][t & 31] = (t >> 5) == (t & 31) ? 1.0 : 0.0;
+        __syncthreads();
+#pragma unroll
+        for (int h = 0; h < 3; ++h)
+            if (rr[h] >= 0) {
+#pragma unroll 8
+                for (int p = 0; p < PANEL; ++p) sum[h] = fma(Li[p][rr[h]], Lc[cc[h]][p], sum[h]);
+                E[rr[h]][cc[h]] = E[cc[h]][rr[h]] = old[h] - sum[h];
+            }
+        __syncthreads();
+        double row[ROWS_PER_WARP];
+#pragma unroll
+        for (int q = 0; q < ROWS_PER_WARP; ++q) row[q] = E[b0 + 8 * q][a];
+        factor_block(B, band, k1, Pn, row, W, bad, status);
+        return;
+    }
+    double s[ROWS_PER_WARP], v[ROWS_PER_WARP];
+    bool on[ROWS_PER_WARP];
+#pragma unroll
+    for (int q = 0; q < ROWS_PER_WARP; ++q) {
+        const int c = c0 + b0 + 8 * q;
+        on[q] = c < e && i >= c && i < e && i - c <= bw;
+        v[q] = on[q] ? A[(int64_t)c * ld + (i - c)] : 0.0;
+        s[q] = 0.0;
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int p = 0; p < PANEL; ++p) {
+        const double li = Li[p][a];
+#pragma unroll
+        for (int q = 0; q < ROWS_PER_WARP; ++q) s[q] = fma(li, Lc[b0 + 8 * q][p], s[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < ROWS_PER_WARP; ++q) {
+        const int c = c0 + b0 + 8 * q;
+        if (on[q]) A[(int64_t)c * ld + (i - c)] = v[q] - s[q];
     }
 }
 
-// x <- (L D L^T)^-1 x, in place, one CTA of 32 warps.
-__global__ void __launch_bounds__(SOLVE_THREADS) k_ldl_solve(int n, int bw, const double *__restrict__ band,
-                                                             double *__restrict__ x)
+// The second band's updates of the middle rows are added to the first band's
+// (first column of the middle: n1; row i of the order is row n - 1 - i there).
+__global__ void k_ldl_merge(int n, int n1, int m, Bands B, const int *status)
 {
-    __shared__ double yb[32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t ld = (int64_t)bw + 1;
-    // forward: L y = x (unit lower), blocks of 32 equations in order
-    for (int kb = 0; kb < n; kb += 32) {
-        const int nbk = min(32, n - kb);
-        if (warp == 0) {
-            double y = lane < nbk ? x[kb + lane] : 0.0;
-            for (int jj = 0; jj < nbk; ++jj) {
-                const double yj = __shfl_sync(0xffffffffu, y, jj);
-                if (lane > jj && lane < nbk && lane - jj <= bw) y -= band[(int64_t)(kb + jj) * ld + (lane - jj)] * yj;
-            }
-            if (lane < nbk) {
-                x[kb + lane] = y;
-                yb[lane] = y;
-            }
-        }
-        __syncthreads();
-        const int64_t iend = min((int64_t)n, (int64_t)kb + nbk + bw);
-        for (int64_t i = (int64_t)kb + nbk + threadIdx.x; i < iend; i += blockDim.x) {
-            double s = 0.0;
-            for (int jj = 0; jj < nbk; ++jj) {
-                const int64_t off = i - (kb + jj);
-                if (off <= bw) s += band[(int64_t)(kb + jj) * ld + off] * yb[jj];
-            }
-            x[i] -= s;
-        }
-        __syncthreads();
+    if (*status) return;
+    const int64_t ld = (int64_t)B.bw + 1;
+    const int j = n1 + blockIdx.x;
+    for (int o = threadIdx.x; o < ld && j + o < n1 + m; o += blockDim.x)
+        B.a[0][(int64_t)j * ld + o] += B.a[1][(int64_t)(n - 1 - (j + o)) * ld + o];
+}
+
+// ---------------------------------------------------------------- substitution
+// L y = x (forward) or L^T x = D^-1 y (backward) over the columns [kb0, kb1) of
+// each band, a thread-block cluster per band. Block by block of 32 equations: every
+// CTA applies the block's stored inverse to its right-hand side (no 32-step chain),
+// then the 32-row tiles of the band below are dealt over the cluster's CTAs: the
+// forward sweep subtracts a tile's product from the rows its CTA owns and hands the
+// next block's rows to all CTAs through distributed shared memory; in the backward
+// sweep the CTAs exchange their tiles' partial sums of the block's columns. One
+// cluster barrier per block. One CTA per system without the inverses took 66 us per
+// block (natural order, half bandwidth 2,567).
+constexpr int SOLVE_CLUSTER = 8;
+
+struct SolveVec {
+    double *x[2];
+};
+
+__device__ __forceinline__ uint32_t cta_rank()
+{
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n"
+                 "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+// v to the same shared-memory word of CTA q of the cluster.
+__device__ __forceinline__ void store_to_cta(double *word, uint32_t q, double v)
+{
+    uint32_t ra;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(ra)
+                 : "r"((uint32_t)__cvta_generic_to_shared(word)), "r"(q));
+    asm volatile("st.relaxed.cluster.shared::cluster.f64 [%0], %1;" ::"r"(ra), "d"(v) : "memory");
+}
+
+// The thread's four entries of a block's 32 x 32 inverse M (transposed with TR): row
+// threadIdx / 8, columns threadIdx % 8 + 8 k; loaded a step ahead.
+template <bool TR>
+__device__ __forceinline__ void block_load(const double *__restrict__ M, double (&m)[4])
+{
+    const int row = threadIdx.x >> 3, part = threadIdx.x & 7;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int c = part + 8 * k;
+        m[k] = __ldg(M + (TR ? c * PANEL + row : row * PANEL + c));
     }
-    // diagonal
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) x[i] = x[i] / band[i * ld];
+}
+
+// out[row] = sum_c M(row, c) in[c]. Valid after the __syncthreads at the end.
+__device__ __forceinline__ void block_times(const double (&m)[4], const double *in, double *out)
+{
+    const int row = threadIdx.x >> 3, part = threadIdx.x & 7;
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) s = fma(m[k], in[part + 8 * k], s);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (part == 0) out[row] = s;
     __syncthreads();
-    // backward: L^T x = y (unit upper), blocks of 32 equations from the end
-    const int last = ((n - 1) / 32) * 32;
-    for (int kb = last; kb >= 0; kb -= 32) {
-        const int nbk = min(32, n - kb);
-        if (warp < nbk) {
-            const int64_t j = kb + warp;
-            const int64_t iend = min((int64_t)n - 1, j + bw);
-            double s = 0.0;
-            for (int64_t i = (int64_t)kb + nbk + lane; i <= iend; i += 32) s += band[j * ld + (i - j)] * x[i];
-            s = warp_sum(s);
-            if (lane == 0) yb[warp] = x[j] - s;
+}
+
+// Tiles of a step whose entries are loaded before the step's barrier (a thread has
+// four entries of a tile); further tiles of wide bands are loaded when they are used.
+constexpr int AHEAD = 3;
+
+// First tile row above k that belongs to CTA `rank`.
+__device__ __forceinline__ int first_tile(int k, int rank)
+{
+    return k + 1 + (rank - (k + 1) % SOLVE_CLUSTER + SOLVE_CLUSTER) % SOLVE_CLUSTER;
+}
+
+// Forward: ring holds the running right-hand sides of the tile rows this CTA owns.
+__global__ void __launch_bounds__(NTHREADS) k_ldl_forward(Bands B, SolveVec V, int kb0, int kb1, int ring)
+{
+    extern __shared__ double own[];            // [ring][32]
+    __shared__ double rhs[2][PANEL], y[PANEL], red[AHEAD][NTHREADS / 32][PANEL];
+    const int band = blockIdx.x / SOLVE_CLUSTER, bw = B.bw, N = B.N[band];
+    const int rank = (int)cta_rank();
+    const double *A = B.a[band];
+    double *x = V.x[band];
+    const int64_t ld = (int64_t)bw + 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x < PANEL) rhs[0][lane] = kb0 + lane < N ? x[kb0 + lane] : 0.0;
+    int seen = kb0 / 32 + 1;   // tile rows from here on still have their right-hand side in x
+    const auto window = [&](int kb) { return (int)min((int64_t)(N - 1) / 32, ((int64_t)min(kb + 32, N) - 1 + bw) / 32); };
+    // entries of tile row t for the block at kb: row t * 32 + lane, columns 4 warp + q
+    const auto load = [&](int kb, int t, double (&v)[4]) {
+        const int i = t * 32 + lane, P = min(32, N - kb);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int j = kb + warp * 4 + q, off = i - j;
+            v[q] = i < N && j < kb + P && off <= bw ? __ldg(A + (int64_t)j * ld + off) : 0.0;
         }
+    };
+    double m[4], v[AHEAD][4], xin[AHEAD];   // xin (warp h < AHEAD): right-hand side of a tile row entering the window
+    const auto ahead = [&](int kb, int from) {
+        block_load<false>(B.xinv[band] + (int64_t)kb * PANEL, m);
+        const int k = kb / 32, last = window(kb);
+#pragma unroll
+        for (int h = 0; h < AHEAD; ++h) {
+            const int t = first_tile(k, rank) + h * SOLVE_CLUSTER;
+            xin[h] = 0.0;
+            if (t > last) continue;
+            load(kb, t, v[h]);
+            if (warp == h && t >= from && t * 32 + lane < N) xin[h] = x[t * 32 + lane];
+        }
+    };
+    ahead(kb0, seen);
+    cluster_sync();
+    for (int kb = kb0, par = 0; kb < kb1; kb += 32, par ^= 1) {
+        const int k = kb / 32, P = min(32, N - kb), last = window(kb);
+        double *rn = rhs[par ^ 1];
+        block_times(m, rhs[par], y);
+        if (rank == 0 && threadIdx.x < P) x[kb + lane] = y[lane];
+        double y4[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) y4[q] = y[warp * 4 + q];
+        const int t0 = first_tile(k, rank);
+        for (int tb = t0; tb <= last; tb += AHEAD * SOLVE_CLUSTER) {
+#pragma unroll
+            for (int h = 0; h < AHEAD; ++h) {
+                const int t = tb + h * SOLVE_CLUSTER;
+                if (t > last) continue;
+                if (tb != t0) load(kb, t, v[h]);
+                red[h][warp][lane] = fma(v[h][0], y4[0], v[h][1] * y4[1]) + fma(v[h][2], y4[2], v[h][3] * y4[3]);
+            }
+            __syncthreads();
+#pragma unroll
+            for (int h = 0; h < AHEAD; ++h) {
+                const int t = tb + h * SOLVE_CLUSTER;
+                if (warp != h || t > last) continue;
+                double *o = own + (size_t)(t / SOLVE_CLUSTER % ring) * PANEL + lane;
+                double r = t < seen ? *o : tb == t0 ? xin[h] : t * 32 + lane < N ? x[t * 32 + lane] : 0.0;
+                r -= ((red[h][0][lane] + red[h][1][lane]) + (red[h][2][lane] + red[h][3][lane])) +
+                     ((red[h][4][lane] + red[h][5][lane]) + (red[h][6][lane] + red[h][7][lane]));
+                *o = r;
+                if (t == k + 1)
+                    for (uint32_t q = 0; q < SOLVE_CLUSTER; ++q) store_to_cta(rn + lane, q, r);
+            }
+            if (tb + AHEAD * SOLVE_CLUSTER <= last) __syncthreads();
+        }
+        if (last < k + 1 && k + 1 <= (N - 1) / 32 && rank == 0 && threadIdx.x < PANEL) {
+            // bw = 0: nothing reaches the next block, its rows go on as they came
+            const int i = (k + 1) * 32 + lane;
+            const double r = i < N ? x[i] : 0.0;
+            for (uint32_t q = 0; q < SOLVE_CLUSTER; ++q) store_to_cta(rn + lane, q, r);
+        }
+        seen = max(seen, last + 1);
+        if (kb + 32 < kb1) ahead(kb + 32, seen);
+        cluster_sync();
+    }
+    // right-hand sides of the rows the range did not eliminate
+    for (int t = kb1 / 32; t < seen; ++t)
+        if (t % SOLVE_CLUSTER == rank && kb1 < N && threadIdx.x < PANEL && t * 32 + lane < N)
+            x[t * 32 + lane] = own[(size_t)(t / SOLVE_CLUSTER % ring) * PANEL + lane];
+}
+
+// Backward: x holds y on entry and the solution on return; the CTA keeps the
+// solution of the tile rows it owns.
+__global__ void __launch_bounds__(NTHREADS) k_ldl_backward(Bands B, SolveVec V, int kb0, int kb1, int ring)
+{
+    extern __shared__ double own[];            // [ring][32]: solution of the owned tile rows
+    __shared__ double part[2][SOLVE_CLUSTER][PANEL], w[PANEL], xk[PANEL], red[NTHREADS / 32][PANEL];
+    const int band = blockIdx.x / SOLVE_CLUSTER, bw = B.bw, N = B.N[band];
+    const int rank = (int)cta_rank();
+    const double *A = B.a[band];
+    double *x = V.x[band];
+    const int64_t ld = (int64_t)bw + 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int kfirst = (kb1 - 1) / 32, klast = kb0 / 32;
+    // tile rows below the range that its columns reach
+    const int deep = (int)min((int64_t)(N - 1) / 32, ((int64_t)kb1 - 1 + bw) / 32);
+    for (int t = kfirst + 1; t <= deep; ++t)
+        if (t % SOLVE_CLUSTER == rank && threadIdx.x < PANEL)
+            own[(size_t)(t / SOLVE_CLUSTER % ring) * PANEL + lane] = t * 32 + lane < N ? x[t * 32 + lane] : 0.0;
+    const auto window = [&](int kb) { return (int)min((int64_t)(N - 1) / 32, ((int64_t)min(kb + 32, N) - 1 + bw) / 32); };
+    // entries of tile row t for the block at kb: lane = column, rows 4 warp + q
+    const auto load = [&](int kb, int t, double (&v)[4]) {
+        const int j = kb + lane, P = min(32, N - kb);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int i = t * 32 + warp * 4 + q;
+            v[q] = i < N && lane < P && i - j <= bw ? __ldg(A + (int64_t)j * ld + (i - j)) : 0.0;
+        }
+    };
+    double m[4], v[AHEAD][4], yd = 0.0;
+    const auto ahead = [&](int k) {
+        const int kb = 32 * k, last = window(kb);
+        block_load<true>(B.xinv[band] + (int64_t)kb * PANEL, m);
+        yd = warp == 0 && kb + lane < N ? x[kb + lane] / __ldg(A + (int64_t)(kb + lane) * ld) : 0.0;
+#pragma unroll
+        for (int h = 0; h < AHEAD; ++h) {
+            const int t = first_tile(k, rank) + h * SOLVE_CLUSTER;
+            if (t <= last) load(kb, t, v[h]);
+        }
+    };
+    ahead(kfirst);
+    cluster_sync();
+    for (int k = kfirst; k >= klast; --k) {
+        const int kb = 32 * k, P = min(32, N - kb), buf = k & 1, last = window(kb);
+        double s = 0.0;
+        const int t0 = first_tile(k, rank);
+        for (int tb = t0; tb <= last; tb += AHEAD * SOLVE_CLUSTER) {
+#pragma unroll
+            for (int h = 0; h < AHEAD; ++h) {
+                const int t = tb + h * SOLVE_CLUSTER;
+                if (t > last) continue;
+                if (tb != t0) load(kb, t, v[h]);
+                const double *o = own + (size_t)(t / SOLVE_CLUSTER % ring) * PANEL + warp * 4;
+                s += fma(v[h][0], o[0], v[h][1] * o[1]) + fma(v[h][2], o[2], v[h][3] * o[3]);
+            }
+        }
+        red[warp][lane] = s;
+        const double y = yd;
+        double mk[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) mk[q] = m[q];
+        if (k > klast) ahead(k - 1);   // (x above block k is not written in this step)
         __syncthreads();
         if (warp == 0) {
-            double v = lane < nbk ? yb[lane] : 0.0;
-            for (int jj = nbk - 1; jj >= 0; --jj) {
-                const double xj = __shfl_sync(0xffffffffu, v, jj);
-                if (lane < jj && jj - lane <= bw) v -= band[(int64_t)(kb + lane) * ld + (jj - lane)] * xj;
-            }
-            if (lane < nbk) x[kb + lane] = v;
+            const double r = ((red[0][lane] + red[1][lane]) + (red[2][lane] + red[3][lane])) +
+                             ((red[4][lane] + red[5][lane]) + (red[6][lane] + red[7][lane]));
+            for (uint32_t q = 0; q < SOLVE_CLUSTER; ++q) store_to_cta(&part[buf][rank][lane], q, r);
+        }
+        cluster_sync();
+        if (warp == 0) {
+            const double(&pp)[SOLVE_CLUSTER][PANEL] = part[buf];
+            w[lane] = y - (((pp[0][lane] + pp[1][lane]) + (pp[2][lane] + pp[3][lane])) +
+                           ((pp[4][lane] + pp[5][lane]) + (pp[6][lane] + pp[7][lane])));
         }
         __syncthreads();
+        block_times(mk, w, xk);
+        if (k % SOLVE_CLUSTER == rank && threadIdx.x < PANEL) {
+            own[(size_t)(k / SOLVE_CLUSTER % ring) * PANEL + lane] = xk[lane];
+            if (lane < P) x[kb + lane] = xk[lane];
+        }
+        __syncthreads();   // (part is double-buffered: one cluster barrier per block)
     }
+}
+
+// b in the order (pos of equation i), split over the two bands' vectors.
+__global__ void k_ldl_scatter(int n, int mid, int m, const int *__restrict__ pos, const double *__restrict__ b, SolveVec V)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int p = pos ? pos[i] : i;
+    if (p < mid) V.x[0][p] = b[i];
+    else V.x[1][n - 1 - p] = b[i];
+    // the middle rows of the second band collect its updates from zero
+    if (V.x[1] && p >= mid - m && p < mid) V.x[1][n - 1 - p] = 0.0;
+}
+
+// Middle rows: to = first band's += second band's (ADD), or second = first.
+template <bool ADD>
+__global__ void k_ldl_middle(int n, int n1, int m, SolveVec V)
+{
+    const int i = n1 + blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n1 + m) return;
+    if (ADD) V.x[0][i] += V.x[1][n - 1 - i];
+    else V.x[1][n - 1 - i] = V.x[0][i];
+}
+
+__global__ void k_ldl_gather(int n, int mid, const int *__restrict__ pos, SolveVec V, double *__restrict__ x)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int p = pos ? pos[i] : i;
+    x[i] = p < mid ? V.x[0][p] : V.x[1][n - 1 - p];
 }
 
 // ||b - y||^2 and ||b||^2 over the first n rows (y = A x), deterministic.
@@ -276,6 +616,222 @@ __global__ void __launch_bounds__(NTHREADS) k_ldl_resid(int64_t n, const double 
 
 }  // namespace
 
+// Half bandwidth of the compressed graph (ptr, adj; size[s] equations of node s)
+// when its nodes are numbered in the given order.
+static int order_bandwidth(const std::vector<int> &order, const std::vector<int> &size, const std::vector<int64_t> &ptr,
+                           const std::vector<int> &adj)
+{
+    const int ns = (int)order.size();
+    std::vector<int> first(ns), last(ns);
+    int at = 0, bw = 0;
+    for (int s : order) {
+        first[s] = at;
+        at += size[s];
+        last[s] = at - 1;
+    }
+    for (int s = 0; s < ns; ++s) {
+        bw = std::max(bw, size[s] - 1);
+        for (int64_t e = ptr[s]; e < ptr[s + 1]; ++e) bw = std::max(bw, last[adj[e]] - first[s]);
+    }
+    return bw;
+}
+
+// A numbering of m's equations with a small half bandwidth: F.pos (position of each
+// equation) and F.bwp, or the natural order. Host work, once per structure; equations
+// with equal rows (a node's) are numbered together, on a graph of a ninth of the
+// entries. Per component the nodes are put in breadth-first levels from one end: the
+// last level of a search from a far node (on a beam that is the whole end face,
+// where a search from one corner node grows into the beam as a cube, with three times
+// the bandwidth). Within the levels they keep the matrix's order or take the order in which
+// the search meets them (Cuthill-McKee), whichever gives the smaller half bandwidth;
+// the natural order stays unless it is beaten. Below ORDER_MIN_BW a panel's trailing
+// update is a few tiles either way and the chain of panels, which no order shortens,
+// is the cost.
+constexpr int ORDER_MIN_BW = 64;
+static int ldl_order(ogb_mtrx *m)
+{
+    LdlFactor &F = m->ldl;
+    cudaStream_t s = m->ctx->stream;
+    const int n = m->neq;
+    F.ordered = false;
+    F.bwp = F.bw;
+    F.order_structure = m->structure;
+    if (F.bw < ORDER_MIN_BW) return OGB_OK;
+    std::vector<int64_t> rp(n + 1);
+    OGB_CUDA(cudaMemcpyAsync(rp.data(), m->rowptr.p, (n + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    OGB_CUDA(cudaStreamSynchronize(s));
+    std::vector<int> ci(rp[n]);
+    OGB_CUDA(cudaMemcpyAsync(ci.data(), m->colind.p, rp[n] * sizeof(int), cudaMemcpyDeviceToHost, s));
+    OGB_CUDA(cudaStreamSynchronize(s));
+    // runs of consecutive equations with equal rows
+    std::vector<int> node(n), size, rep;
+    for (int i = 0; i < n; ++i) {
+        const int64_t len = rp[i + 1] - rp[i];
+        if (i > 0 && len == rp[i] - rp[i - 1] && std::equal(ci.begin() + rp[i], ci.begin() + rp[i + 1], ci.begin() + rp[i - 1])) {
+            node[i] = node[i - 1];
+            size[node[i]]++;
+        } else {
+            node[i] = (int)size.size();
+            size.push_back(1);
+            rep.push_back(i);
+        }
+    }
+    const int ns = (int)size.size();
+    std::vector<int64_t> ptr(ns + 1, 0);
+    std::vector<int> adj;
+    for (int q = 0; q < ns; ++q) {
+        int prev = -1;
+        for (int64_t k = rp[rep[q]]; k < rp[rep[q] + 1]; ++k) {
+            if (ci[k] >= n || node[ci[k]] == prev) continue;
+            prev = node[ci[k]];
+            if (prev != q) adj.push_back(prev);
+        }
+        ptr[q + 1] = (int64_t)adj.size();
+    }
+    std::vector<int> mark(ns, -1), by_level, by_search;
+    std::vector<char> placed(ns, 0);
+    int stamp = 0;
+    // breadth-first from `from`: the nodes as met, and the start of every level
+    const auto search = [&](const std::vector<int> &from, std::vector<int> &met, std::vector<int> &lev) {
+        ++stamp;
+        met = from;
+        lev.assign(1, 0);
+        for (int q : from) mark[q] = stamp;
+        for (size_t a = 0, b = met.size(); a < b; b = met.size()) {
+            lev.push_back((int)b);
+            for (; a < b; ++a)
+                for (int64_t e = ptr[met[a]]; e < ptr[met[a] + 1]; ++e)
+                    if (mark[adj[e]] != stamp) {
+                        mark[adj[e]] = stamp;
+                        met.push_back(adj[e]);
+                    }
+        }
+    };
+    std::vector<int> met, lev;
+    for (int root = 0; root < ns; ++root) {
+        if (placed[root]) continue;
+        search({root}, met, lev);
+        for (int pass = 0; pass < 3; ++pass) {   // a node far from everything: the last level's of least degree
+            const size_t depth = lev.size();
+            int far = met.back();
+            for (size_t k = lev[lev.size() - 2]; k < met.size(); ++k)
+                if (ptr[met[k] + 1] - ptr[met[k]] < ptr[far + 1] - ptr[far]) far = met[k];
+            search({far}, met, lev);
+            if (lev.size() <= depth) break;
+        }
+        std::vector<int> end(met.begin() + lev[lev.size() - 2], met.end());
+        std::sort(end.begin(), end.end());
+        search(end, met, lev);
+        by_search.insert(by_search.end(), met.begin(), met.end());
+        for (size_t k = 0; k + 1 < lev.size(); ++k) std::sort(met.begin() + lev[k], met.begin() + lev[k + 1]);
+        by_level.insert(by_level.end(), met.begin(), met.end());
+        for (int q : met) placed[q] = 1;
+    }
+    if ((int)by_level.size() != ns) return OGB_OK;   // not a symmetric pattern: no order from it
+    const int bl = order_bandwidth(by_level, size, ptr, adj), bs = order_bandwidth(by_search, size, ptr, adj);
+    if (std::min(bl, bs) >= F.bw) return OGB_OK;
+    const std::vector<int> &order = bl <= bs ? by_level : by_search;
+    std::vector<int> pos(n);
+    int at = 0;
+    for (int q : order)
+        for (int k = 0; k < size[q]; ++k) pos[rep[q] + k] = at++;
+    OGB_CHECK(F.pos.alloc(n));
+    OGB_CUDA(cudaMemcpyAsync(F.pos.p, pos.data(), n * sizeof(int), cudaMemcpyHostToDevice, s));
+    OGB_CUDA(cudaStreamSynchronize(s));
+    F.bwp = std::min(bl, bs);
+    F.ordered = true;
+    return OGB_OK;
+}
+
+static Bands ldl_bands(const LdlFactor &F)
+{
+    Bands B{};
+    const int64_t ld = (int64_t)F.bwf + 1;
+    const int64_t x0 = ceil_div(F.n1 + F.mid, PANEL) * PANEL * PANEL;
+    B.bw = F.bwf;
+    B.N[0] = F.n1 + F.mid;
+    B.a[0] = F.band.p;
+    B.xinv[0] = F.xinv.p;
+    if (F.n1) {
+        B.N[1] = F.n1 + F.mid;
+        B.a[1] = F.band.p + (int64_t)B.N[0] * ld;
+        B.xinv[1] = F.xinv.p + x0;
+    }
+    return B;
+}
+
+// Factor in the chosen order (natural: as the equations come, from one end).
+static int ldl_factor_in(ogb_mtrx *m, bool natural, int *pivot)
+{
+    LdlFactor &F = m->ldl;
+    ogb_ctx *ctx = m->ctx;
+    cudaStream_t s = ctx->stream;
+    const int n = m->neq;
+    const int bw = natural ? F.bw : F.bwp;
+    F.use_pos = !natural && F.ordered;
+    // equal ends in whole panels around at least bw middle rows
+    F.n1 = natural ? 0 : std::max(0, (n - bw) / 64 * PANEL);
+    F.mid = n - 2 * F.n1;
+    F.bwf = bw;
+    const int64_t ld = (int64_t)bw + 1;
+    const size_t need = (size_t)(F.n1 ? n + F.mid : n) * (size_t)ld;
+    if (F.band.n < need) {
+        size_t freeb = 0, total = 0;
+        OGB_CUDA(cudaMemGetInfo(&freeb, &total));
+        const size_t have = F.band.n * sizeof(double);
+        if (need * sizeof(double) > (freeb + have) / 10 * 9)
+            return fail(OGB_E_LIMIT, "direct solver: the band of " + std::to_string(n) + " x " + std::to_string(ld) +
+                                         " doubles does not fit in device memory");
+    }
+    OGB_CHECK(F.band.alloc(need));
+    OGB_CHECK(F.xinv.alloc((size_t)2 * ceil_div(F.n1 + F.mid, PANEL) * PANEL * PANEL));
+    const Bands B = ldl_bands(F);
+    OGB_CUDA(cudaMemsetAsync(F.band.p, 0, need * sizeof(double), s));
+    int *st = F.d_int.p + 1;
+    OGB_CUDA(cudaMemsetAsync(st, 0, sizeof(int), s));
+    k_ldl_fill<<<(unsigned)ceil_div((int64_t)n * 32, NTHREADS), NTHREADS, 0, s>>>(
+        n, F.n1 + F.mid, m->rowptr.p, m->colind.p, m->val.p, F.use_pos ? F.pos.p : nullptr, B);
+    count_launch(ctx);
+    static bool tdone[64] = {};
+    OGB_CUDA(set_smem_limit_once((const void *)k_ldl_trailing, EXCLUSIVE_SMEM, tdone));
+    auto panels = [&](int kb0, int kb1, int nb) {
+        if (kb0 >= kb1) return;
+        k_ldl_diag<<<nb, NTHREADS, 0, s>>>(B, kb0, st);
+        count_launch(ctx);
+        for (int k0 = kb0; k0 < kb1; k0 += PANEL) {
+            const int k1 = std::min(k0 + PANEL, B.N[0]);
+            const int e = (int)std::min<int64_t>((int64_t)B.N[0], (int64_t)k1 + bw);
+            if (e <= k1) {   // bw = 0: no rows below; the next block as it stands
+                if (k1 < kb1) {
+                    k_ldl_diag<<<nb, NTHREADS, 0, s>>>(B, k1, st);
+                    count_launch(ctx);
+                }
+                continue;
+            }
+            k_ldl_subpanel<<<dim3((unsigned)ceil_div(e - k1, SUB_ROWS), nb), NTHREADS, 0, s>>>(B, k0, st);
+            const unsigned nt = (unsigned)ceil_div(e - k1, 32);
+            // few tiles: one CTA per SM (by its shared memory), so that no tile shares
+            // the FP64 pipe of the CTA that factors the next block, the longest of
+            // the launch (60 x 12 x 12 hexes: 32.7 us against 44.8 us); from four per SM on the
+            // tiles take longer than that block, and several per SM hide their loads
+            const size_t excl = (int64_t)(nt * (nt + 1) / 2) * nb <= 4 * (int64_t)num_sms() ? EXCLUSIVE_SMEM : 0;
+            k_ldl_trailing<<<nt * (nt + 1) / 2 * nb, NTHREADS, excl, s>>>(B, nb, k0, k1 < kb1 ? 1 : 0, st);
+            count_launch(ctx, 2);
+        }
+    };
+    if (F.n1) {
+        panels(0, F.n1, 2);
+        k_ldl_merge<<<F.mid, NTHREADS, 0, s>>>(n, F.n1, F.mid, B, st);
+        count_launch(ctx);
+    }
+    panels(F.n1, B.N[0], 1);
+    OGB_CUDA(cudaGetLastError());
+    OGB_CUDA(cudaMemcpyAsync(F.h_int.p + 1, st, sizeof(int), cudaMemcpyDeviceToHost, s));
+    OGB_CUDA(cudaStreamSynchronize(s));
+    *pivot = F.h_int.p[1];
+    return OGB_OK;
+}
+
 // Factor m's current values (cached per matrix version).
 int ldl_factor(ogb_mtrx *m)
 {
@@ -287,54 +843,76 @@ int ldl_factor(ogb_mtrx *m)
     F.ok = false;
     OGB_CHECK(F.d_int.alloc(2));
     OGB_CHECK(F.h_int.alloc(2));
-    OGB_CUDA(cudaMemsetAsync(F.d_int.p, 0, 2 * sizeof(int), s));
-    if (n > 0) {
-        k_ldl_bandwidth<<<nblk(n), NTHREADS, 0, s>>>(n, m->rowptr.p, m->colind.p, F.d_int.p);
-        count_launch(ctx);
-    }
-    OGB_CUDA(cudaMemcpyAsync(F.h_int.p, F.d_int.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    OGB_CUDA(cudaStreamSynchronize(s));
-    const int bw = F.h_int.p[0];
-    const int64_t ld = (int64_t)bw + 1;
-    const size_t need = (size_t)n * (size_t)ld;
-    if (F.band.n < need) {
-        size_t freeb = 0, total = 0;
-        OGB_CUDA(cudaMemGetInfo(&freeb, &total));
-        const size_t have = F.band.n * sizeof(double);
-        if (need * sizeof(double) > (freeb + have) / 10 * 9)
-            return fail(OGB_E_LIMIT, "direct solver: the band of " + std::to_string(n) + " x " + std::to_string(ld) +
-                                         " doubles does not fit in device memory");
-    }
-    OGB_CHECK(F.band.alloc(need));
-    F.n = n;
-    F.bw = bw;
-    if (n > 0) {
-        OGB_CUDA(cudaMemsetAsync(F.band.p, 0, need * sizeof(double), s));
-        k_ldl_fill<<<(unsigned)ceil_div((int64_t)n * 32, NTHREADS), NTHREADS, 0, s>>>(n, bw, m->rowptr.p, m->colind.p,
-                                                                                        m->val.p, F.band.p);
-        count_launch(ctx);
-        int *st = F.d_int.p + 1;
-        for (int k0 = 0; k0 < n; k0 += PANEL) {
-            const int k1 = k0 + PANEL < n ? k0 + PANEL : n;
-            k_ldl_diag<<<1, PANEL_THREADS, 0, s>>>(n, bw, F.band.p, k0, k1, st);
+    if (F.order_structure != m->structure || F.n != n) {
+        F.n = n;
+        OGB_CUDA(cudaMemsetAsync(F.d_int.p, 0, 2 * sizeof(int), s));
+        if (n > 0) {
+            k_ldl_bandwidth<<<nblk(n), NTHREADS, 0, s>>>(n, m->rowptr.p, m->colind.p, F.d_int.p);
             count_launch(ctx);
-            const int e = (int)std::min<int64_t>((int64_t)n, (int64_t)k1 + bw);
-            if (e > k1) {
-                k_ldl_subpanel<<<(unsigned)ceil_div(e - k1, NTHREADS), NTHREADS, 0, s>>>(n, bw, F.band.p, k0, k1, st);
-                const unsigned nt = (unsigned)ceil_div(e - k1, 32);
-                k_ldl_trailing<<<dim3(nt, nt), NTHREADS, 0, s>>>(n, bw, F.band.p, k0, k1, st);
-                count_launch(ctx, 2);
-            }
         }
-        OGB_CUDA(cudaGetLastError());
+        OGB_CUDA(cudaMemcpyAsync(F.h_int.p, F.d_int.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+        OGB_CUDA(cudaStreamSynchronize(s));
+        F.bw = F.h_int.p[0];
+        OGB_CHECK(ldl_order(m));
     }
-    OGB_CUDA(cudaMemcpyAsync(F.h_int.p + 1, F.d_int.p + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
-    OGB_CUDA(cudaStreamSynchronize(s));
-    if (F.h_int.p[1] != 0)
-        return fail(OGB_E_ZERODIAG, "direct solver: zero or non-finite pivot at equation " +
-                                        std::to_string(F.h_int.p[1]));
+    if (n > 0) {
+        int pivot = 0;
+        OGB_CHECK(ldl_factor_in(m, false, &pivot));
+        if (pivot != 0 && (F.use_pos || F.n1 > 0)) OGB_CHECK(ldl_factor_in(m, true, &pivot));
+        if (pivot != 0)
+            return fail(OGB_E_ZERODIAG, "direct solver: zero or non-finite pivot at equation " + std::to_string(pivot));
+    }
     F.version = m->version;
     F.ok = true;
+    return OGB_OK;
+}
+
+// x = A^-1 b with the factor, over the first n equations.
+static int ldl_substitute(ogb_mtrx *m, const double *b, double *x)
+{
+    LdlFactor &F = m->ldl;
+    cudaStream_t s = m->ctx->stream;
+    const int n = F.n, N = F.n1 + F.mid;
+    const Bands B = ldl_bands(F);
+    OGB_CHECK(F.xv.alloc((size_t)2 * N));
+    SolveVec V{{F.xv.p, F.n1 ? F.xv.p + N : nullptr}};
+    const int *pos = F.use_pos ? F.pos.p : nullptr;
+    const int ring = (int)((F.bwf / 32 + 2) / SOLVE_CLUSTER + 2);
+    const size_t smem = (size_t)ring * PANEL * sizeof(double);
+    static bool fdone[64] = {}, bdone[64] = {};
+    // (a band whose ring would not fit this limit is larger than device memory)
+    OGB_CUDA(set_smem_limit_once((const void *)k_ldl_forward, 200 * 1024, fdone));
+    OGB_CUDA(set_smem_limit_once((const void *)k_ldl_backward, 200 * 1024, bdone));
+    auto sweep = [&](bool fwd, int kb0, int kb1, int nb) -> int {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(nb * SOLVE_CLUSTER);
+        cfg.blockDim = dim3(NTHREADS);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = SOLVE_CLUSTER;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        OGB_CUDA(cudaLaunchKernelEx(&cfg, fwd ? k_ldl_forward : k_ldl_backward, B, V, kb0, kb1, ring));
+        return OGB_OK;
+    };
+    k_ldl_scatter<<<nblk(n), NTHREADS, 0, s>>>(n, N, F.n1 ? F.mid : 0, pos, b, V);
+    if (F.n1) {
+        OGB_CHECK(sweep(true, 0, F.n1, 2));
+        k_ldl_middle<true><<<nblk(F.mid), NTHREADS, 0, s>>>(n, F.n1, F.mid, V);
+    }
+    OGB_CHECK(sweep(true, F.n1, N, 1));
+    OGB_CHECK(sweep(false, F.n1, N, 1));
+    if (F.n1) {
+        k_ldl_middle<false><<<nblk(F.mid), NTHREADS, 0, s>>>(n, F.n1, F.mid, V);
+        OGB_CHECK(sweep(false, 0, F.n1, 2));
+    }
+    k_ldl_gather<<<nblk(n), NTHREADS, 0, s>>>(n, N, pos, V, x);
+    count_launch(m->ctx, F.n1 ? 8 : 4);
+    OGB_CUDA(cudaGetLastError());
     return OGB_OK;
 }
 
@@ -353,11 +931,7 @@ int ldl_solve(ogb_mtrx *m, const double *b, double *x, ogb_solve_info *info)
     OGB_CHECK(r);
     LdlFactor &F = m->ldl;
     if (x != b) OGB_CUDA(cudaMemcpyAsync(x, b, (size_t)m->npad * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    if (F.n > 0) {
-        k_ldl_solve<<<1, SOLVE_THREADS, 0, s>>>(F.n, F.bw, F.band.p, x);
-        count_launch(ctx);
-    }
-    OGB_CUDA(cudaGetLastError());
+    if (F.n > 0) OGB_CHECK(ldl_substitute(m, b, x));
     if (info) {
         const int64_t np = m->npad;
         OGB_CHECK(F.y.alloc(np));

@@ -202,13 +202,21 @@ struct IcFactor {
     bool cluster_local = false;   // ... for the shared-memory form
 };
 
-// LDL^T factor of the direct solver (direct.cu): dense band of n x (bw+1)
-// doubles, column j holds L(j..j+bw, j) with d_j in its diagonal slot.
+// LDL^T factor of the direct solver (direct.cu): dense bands of columns of bwf + 1
+// doubles, column j holds L(j..j+bwf, j) with d_j in its diagonal slot. The first
+// band has n1 + mid rows of the order, the second (n1 > 0) the last n1 + mid,
+// reversed; both eliminate n1 rows, then the first eliminates the middle.
 struct LdlFactor {
     int64_t version = -1;   // matrix version the factor belongs to
     bool ok = false;
-    int n = 0, bw = 0;      // equations, half bandwidth
-    DBuf<double> band;
+    int n = 0, bw = 0;      // equations, half bandwidth in their own order
+    int64_t order_structure = -1;   // matrix structure the order was made for
+    bool ordered = false;   // pos holds a better order, of half bandwidth bwp
+    int bwp = 0;
+    DBuf<int> pos;          // position of each equation
+    bool use_pos = false;   // the factor's own: order, rows per end, middle rows, half bandwidth
+    int n1 = 0, mid = 0, bwf = 0;
+    DBuf<double> band, xinv, xv;   // bands, inverses of the diagonal blocks' triangles, solve vectors
     DBuf<int> d_int;        // [0] half bandwidth, [1] 1-based equation of a zero pivot
     HBuf<int> h_int;
     DBuf<double> y, part, out;   // residual check of a solve
@@ -265,6 +273,7 @@ struct ogb_mtrx {
     int npad = 0;         // rows incl. identity padding (multiple of CHUNK)
     int64_t nnz = 0;      // pattern entries of the neq real rows
     int64_t version = 0;
+    int64_t structure = 0;       // advanced whenever a pattern is built
     bool has_structure = false;
     ogb::DBuf<int64_t> rowptr;   // npad+1
     ogb::DBuf<int> colind;       // nnz + (npad-neq)

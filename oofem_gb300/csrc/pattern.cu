@@ -450,6 +450,7 @@ int build_model_pattern(ogb_model *md, ogb_mtrx *m)
     OGB_CUDA(cudaStreamSynchronize(st));
     OGB_CHECK(check_device_status(ctx, "pattern build"));
     m->has_structure = true;
+    m->structure++;
     m->version++;
     return OGB_OK;
 }
@@ -502,6 +503,7 @@ int build_loc_pattern(ogb_mtrx *m, int neq, int nelem, const int64_t *loc_ptr_h,
     OGB_CUDA(cudaStreamSynchronize(st));
     OGB_CHECK(check_device_status(ctx, "row pattern fill"));
     m->has_structure = true;
+    m->structure++;
     m->version++;
     return OGB_OK;
 }

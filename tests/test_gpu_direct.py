@@ -174,3 +174,72 @@ def test_direct_refactors_after_set_at(ctx, native_lib):
     x2 = A.ldlt_solve(b)
     assert not np.array_equal(x1, x2)
     assert rel(x2, np.linalg.solve(K, b)) < 1e-11
+
+
+@pytest.mark.parametrize("mesh,size", [("hex", (1, 1, 1)), ("hex", (9, 2, 2)), ("hex", (25, 5, 6)), ("hex", (3, 11, 2)),
+                                       ("quad", 1), ("quad", 8), ("quad", 43), ("tet", 3), ("tet", 9)])
+def test_direct_sizes_against_oracle(mesh, size, native_lib, oracle):
+    """The reordered band factored from both ends: no second band (few rows, half
+    bandwidth above half the rows), one panel per end, ragged middles, bands that
+    the natural order already numbers best, and two and three DOFs per node,
+    against the oracle's CG to 1e-14. Both are backward stable: they agree to the
+    condition number (below 1e6 here) times 1e-14, with a margin of ten."""
+    from oofem_gb300 import meshgen as mg
+    if mesh == "hex":
+        m = mg.hex_cantilever(*size, jitter=0.2, seed=3)
+    elif mesh == "quad":
+        m = mg.quad_rve(size, seed=3)
+    else:
+        m = mg.tet_cube_linear(size, jitter=0.15, seed=3)
+    model = native_lib.GpuModel(native_lib.Context(0), m)
+    A = native_lib.GpuCsrMtrx(model.ctx)
+    A.set_solver(native_lib.LS_DIRECT)
+    u, reac, info = model.linear_static(A, rtol=1e-30, maxit=1)
+    assert info.status == 0 and info.achieved < 1e-11, info.achieved
+    ref = oracle.linear_static(oracle.mesh_dict(m), rtol=1e-14)
+    assert rel(u, ref["u"]) < 1e-7, rel(u, ref["u"])
+    # a second factorization of the same structure gives the same bits
+    u2, reac2, _ = model.linear_static(A, rtol=1e-30, maxit=1)
+    assert np.array_equal(u, u2) and np.array_equal(reac, reac2)
+
+
+def assembled(native_lib, n, locs, kes):
+    A = native_lib.GpuCsrMtrx(native_lib.Context(0))
+    A.build_internal_structure(n, locs)
+    A.assemble_begin()
+    K = np.zeros((n, n))
+    for loc, ke in zip(locs, kes):
+        A.assemble(loc, ke)
+        K[np.ix_(loc - 1, loc - 1)] += ke
+    A.assemble_end()
+    return A, K
+
+
+@pytest.mark.parametrize("n", [1, 31, 64, 100, 333])
+def test_direct_drop_in_shuffled_chain(n, native_lib):
+    """Drop-in matrices from location arrays whose own order has a needlessly wide
+    band (a shuffled chain), against numpy."""
+    rng = np.random.default_rng(n)
+    perm = rng.permutation(n)
+    locs = [np.array([perm[i], perm[i + 1]]) + 1 for i in range(n - 1)] + [np.array([perm[n - 1] + 1])]
+    kes = []
+    for loc in locs:
+        g = rng.standard_normal((len(loc), len(loc)))
+        kes.append(g @ g.T + 0.5 * np.eye(len(loc)))
+    A, K = assembled(native_lib, n, locs, kes)
+    b = rng.standard_normal(n)
+    x = A.ldlt_solve(b)
+    assert rel(x, np.linalg.solve(K, b)) < 1e-10
+
+
+def test_direct_zero_pivot_of_the_far_end(native_lib):
+    """A chain whose last diagonal entry is zero: elimination from the first
+    equation meets no zero pivot, elimination from the last one does at once; the
+    matrix is factored from the first equation alone."""
+    n = 300
+    locs = [np.array([i + 1, i + 2]) for i in range(n - 1)]
+    kes = [np.array([[2.0, -1.0], [-1.0, 0.0]]) for _ in locs]
+    A, K = assembled(native_lib, n, locs, kes)
+    assert K[n - 1, n - 1] == 0.0
+    b = np.random.default_rng(1).standard_normal(n)
+    assert rel(A.ldlt_solve(b), np.linalg.solve(K, b)) < 1e-10
