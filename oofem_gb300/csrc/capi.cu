@@ -365,6 +365,12 @@ int64_t ogb_ctx_kernel_launches(ogb_ctx *ctx) { return ctx ? ctx->launches : 0; 
 int ogb_ctx_set_option(ogb_ctx *ctx, int option, int64_t value)
 {
     if (!ctx) return fail(OGB_E_ARG, "null context");
+    switch (option) {   // options that choose a form of the per-iteration launches keep to those launches
+    case OGB_OPT_MIXED_VEC32: case OGB_OPT_MIXED_DIFF: case OGB_OPT_MIXED_P32: case OGB_OPT_MIXED_X64:
+    case OGB_OPT_SPMV_VARIANT: case OGB_OPT_SPMV_HALF: case OGB_OPT_MIXED_BLOCK_JACOBI: case OGB_OPT_UPDATE_BLOCKS:
+    case OGB_OPT_HALF_FORM: case OGB_OPT_FUSED_UPDATE: ctx->persist = false; break;
+    default: break;
+    }
     switch (option) {
     case OGB_OPT_MIXED_VEC32: ctx->mixed_vec32 = value != 0; return OGB_OK;
     case OGB_OPT_MIXED_DIFF: ctx->mixed_diff = value != 0; return OGB_OK;

@@ -162,6 +162,7 @@ struct SellMat {
     int64_t nslots = 0;
     DBuf<int64_t> sl_ptr;   // nslices+1
     DBuf<int> sl_width;     // blocks per row of each slice
+    int max_width = 0;
     DBuf<int> col;          // nslots
     DBuf<int64_t> diag;     // slot of the diagonal block of each row (nslices*32)
     DBuf<double> v64;       // nslots * ND*ND
@@ -261,6 +262,7 @@ struct ogb_ctx {
     bool batch_x64 = false;     // batched mixed solves: FP64 solution every iteration (else FP32 increment per batch)
     int spmv_split = 0;         // warps per slice forced (1, 2, 4) or 0 = the slice-count rule
     double mixed_drop = 0.1;    // residual drop between FP64 replacements
+    bool persist = true;        // iterations of small systems in one launch (persist.cu); off once a form of the per-iteration launches is chosen
     bool mixed_bj = true;       // mixed solves on node-block operators: block-Jacobi preconditioner
     int tangent_tc = 0;         // mixed Newton tangents on tensor cores: 0 never, 1 always, 2 when timed faster
     ogb::DBuf<int> status;           // device status word
@@ -294,6 +296,8 @@ struct ogb_mtrx {
     ogb::DBuf<ogb::PcgScal> w_scal;
     ogb::HBuf<ogb::PcgScal> h_scal;
     ogb::DBuf<unsigned int> w_count;
+    ogb::DBuf<double> w_mail;                    // mailboxes of the one-launch iterations (persist.cu)
+    unsigned long long mail_epoch = 0;           // last exchange posted to them
     ogb::DBuf<unsigned int> w_epoch;             // fused update: advanced once per iteration by its last block
     int spmv_tpr = 8;    // threads per row of the CSR SpMV (autotuned)
     // node-block copy used by the solver when the matrix was built from a model
@@ -417,6 +421,15 @@ int pcg_fp64(ogb_mtrx *m, const double *b, double *x, double rtol, int maxit, og
 int pcg_mixed(ogb_mtrx *m, const double *b, double *x, double rtol, int maxit, ogb_solve_info *info);
 int extract_diag(ogb_mtrx *m);
 int pick_tpr(const ogb_mtrx *m);
+
+// persist.cu: CG iterations of a small node-block system in one launch.
+struct PersistPlan {
+    int rows = 0, grid = 0, nt = 0, rpt = 1, kmax = 0, kc = 0;
+    size_t smem = 0;
+};
+bool persist_plan(const ogb_ctx *ctx, const SellMat &S, bool mixed, PersistPlan &P);
+int persist_run(ogb_mtrx *m, const PersistPlan &P, bool mixed, const void *val, double *x, void *r, void *p, void *z,
+                void *p2, const void *prec, double rtol, int maxit);
 
 // direct.cu: LDL^T factor of m (cached per version) and x = A^-1 b on padded
 // equation-space device vectors (info: 0 iterations, FP64 relative residual).

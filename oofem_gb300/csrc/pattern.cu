@@ -747,7 +747,11 @@ int build_sell(ogb_model *md, ogb_mtrx *m)
     k_ns_of_eq<<<nblk(nn), NTHREADS, 0, st>>>(nn, nd, md->eq.p, md->act.p, S.ns_of_eq.p);
     count_launch(ctx, 2);
     OGB_CUDA(cudaGetLastError());
+    std::vector<int> w(nslices);
+    OGB_CUDA(cudaMemcpyAsync(w.data(), S.sl_width.p, nslices * sizeof(int), cudaMemcpyDeviceToHost, st));
     OGB_CUDA(cudaStreamSynchronize(st));   // the temporaries above are freed on return
+    S.max_width = 0;
+    for (int v : w) S.max_width = v > S.max_width ? v : S.max_width;
     S.v32_version = -1;
     m->has_sell = true;
     return OGB_OK;

@@ -1,0 +1,488 @@
+// CG iterations of small and middle-sized node-block systems in one launch.
+//
+// An iteration of the multi-launch form (solver.cu) is two or three kernels of a few
+// microseconds of latency each: 22-28 us on 10-30 k equations, where the FP64
+// products take 1.5-4 us. Here one cooperative launch runs iterations until the
+// system is done (or a budget of iterations, after which the host looks and launches
+// again). Every CTA owns a share of the node rows for the whole launch:
+//   - its blocks of the matrix stay in shared memory (as many as fit; the rest is
+//     streamed from L2), laid out per thread: four threads share a node row and
+//     take its blocks in turn, so 27-block rows fill warps whatever their number;
+//   - x, r, p and the preconditioner of a degree of freedom stay in the registers
+//     of one of those threads; z and p go to memory for the other CTAs' gathers,
+//     which form z + beta p_old themselves (the same multiply-add as the owner's), so
+//     that no barrier stands between beta and the next product;
+//   - the sums p.q and (r.r, r.z) go through one exchange each (see exchange), which
+//     is reduction and grid barrier at once; every CTA forms the same scalars from
+//     the same values in the same order (bitwise reproducible, no broadcast).
+// Waits are bounded: a mailbox that does not fill within the limit ends the launch
+// with done = 5 in the scalars, as in the fused update.
+//
+// Measured (GB300, per iteration, multi-launch form -> this one): FP64 10.0 k equations
+// 23 -> 12 us, 30.4 k 28 -> 15.5 us; mixed 129 k 33 -> 16.5 us. What is left of the 12 us:
+// products 4.5 (one FP64 instruction of a warp issues in 64 cycles on a quarter of an
+// SM), the two exchanges 2 and 3.5 (the second with its fences), sums and scalars 2.
+//
+// Same arithmetic as the multi-launch form, other sum orders: FP64 (IML CG) with the
+// scalar diagonal, or mixed (FP32 r, z, p, q on the FP32 difference-form copy, FP64
+// x, block Jacobi, leaving on a due residual replacement).
+#include <math.h>
+
+#include <algorithm>
+
+#include "internal.cuh"
+
+namespace ogb {
+
+namespace {
+
+constexpr int PARTS = 4;                  // threads per node row
+constexpr int MAX_CTAS = 160;             // five mailboxes per lane of a warp
+constexpr int PERSIST_SPIN = 1 << 20;     // polls before a wait gives up
+constexpr int WAIT_TIMEOUT = 5;           // PcgScal::done of a wait that gave up
+constexpr int BUDGET = 512;               // iterations of a launch
+constexpr int SMEM_LIMIT = 227 * 1024;
+constexpr int STATIC_SMEM = 12 * 1024;    // the kernels' own shared arrays, rounded up
+
+// A value and the exchange it belongs to, moved as one 16-byte access.
+struct __align__(16) Mail {
+    double value;
+    unsigned long long epoch;
+};
+
+struct PersistArgs {
+    int nrows, rows, kmax, kc;            // node rows; per CTA; blocks per thread, of them in shared memory
+    const int64_t *sl_ptr;
+    const int *sl_width, *col;
+    const void *val;
+    double *x;
+    void *r, *p, *z, *p2;                 // p2: second buffer of p
+    const void *prec;                     // FP64: D^-1 by row; mixed: planes of the block inverses
+    int64_t planes;                       // rows of a plane
+    Mail *mail;                           // [2][receiver][sender][2]
+    unsigned long long epoch;             // of the launch's first exchange
+    PcgScal *sc;
+    double rtol;
+    int maxit;
+};
+
+// The matrix entries of one thread: block k of its row pass, in shared memory or in
+// the SELL copy.
+template <int ND, class T, int RPT>
+struct Blocks {
+    T *sv;
+    int *sc;
+    int nt, kc;
+    __device__ __forceinline__ T *value(int rp, int k, int e) const { return sv + ((size_t)(rp * kc + k) * (ND * ND) + e) * nt + threadIdx.x; }
+    __device__ __forceinline__ int *column(int rp, int k) const { return sc + (size_t)(rp * kc + k) * nt + threadIdx.x; }
+};
+
+__device__ __forceinline__ void post(Mail *m, double v, unsigned long long epoch)
+{
+    const unsigned __int128 b = (unsigned __int128)epoch << 64 | (unsigned long long)__double_as_longlong(v);
+    asm volatile("st.relaxed.gpu.global.b128 [%0], %1;" ::"l"(m), "q"(b) : "memory");
+}
+
+__device__ __forceinline__ bool collect(const Mail *m, double &v, unsigned long long epoch)
+{
+    unsigned __int128 b;
+    asm volatile("ld.relaxed.gpu.global.b128 %0, [%1];" : "=q"(b) : "l"(m) : "memory");
+    v = __longlong_as_double((long long)(unsigned long long)b);
+    return (unsigned long long)(b >> 64) == epoch;
+}
+
+// Grid-wide sums of NV values of every CTA, by its first warp: the CTA posts its
+// value to a mailbox of every CTA and polls its own mailboxes. A mailbox is polled
+// by one CTA only (slots polled by all CTAs took 6 us an exchange), and the value
+// and its epoch travel in one 16-byte access, so nothing is cleared and an exchange
+// of values alone needs no fence. Two sets alternate: a CTA posts exchange n + 2 after
+// it has everyone's n + 1, posted after their senders had read n. ORDER: what any
+// thread of any CTA wrote before is visible to the warp after (and to its CTA after
+// the next __syncthreads). False when a wait gave up.
+template <int NV, bool ORDER>
+__device__ __forceinline__ bool exchange(Mail *mail, unsigned long long epoch, const double (&mine)[NV], double (&sum)[NV])
+{
+    constexpr int PER = MAX_CTAS / 32;
+    const int G = gridDim.x, lane = threadIdx.x & 31;
+    Mail *set = mail + (size_t)(epoch & 1) * 2 * G * G;
+    if (ORDER) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+#pragma unroll
+    for (int k = 0; k < PER; ++k)
+        if (lane + 32 * k < G)
+#pragma unroll
+            for (int v = 0; v < NV; ++v) post(set + ((size_t)(lane + 32 * k) * G + blockIdx.x) * 2 + v, mine[v], epoch);
+    double got[NV][PER];
+    bool all;
+    int spin = 0;
+    do {
+        all = true;
+#pragma unroll
+        for (int k = 0; k < PER; ++k)
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                got[v][k] = 0.0;
+                if (lane + 32 * k < G) all &= collect(set + ((size_t)blockIdx.x * G + lane + 32 * k) * 2 + v, got[v][k], epoch);
+            }
+        all = __all_sync(0xffffffffu, all);
+    } while (!all && ++spin < PERSIST_SPIN);
+    if (ORDER) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+#pragma unroll
+    for (int v = 0; v < NV; ++v) sum[v] = ((got[v][0] + got[v][1]) + (got[v][2] + got[v][3])) + got[v][4];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int v = 0; v < NV; ++v) sum[v] += __shfl_xor_sync(0xffffffffu, sum[v], o);
+    return all;
+}
+
+// Fixed-order sums over the CTA of NV values per thread held in `in` (count entries
+// each, `stride` apart), for the first warp. Up to four warps per value, so that the
+// FP64 additions of a thousand values do not queue up in every warp's shuffles.
+template <int NV, class T>
+__device__ __forceinline__ void cta_sum(const T *in, int count, int stride, double (&out)[NV], double *warp_sums)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int per = nw >= 4 * NV ? 4 : nw >= NV ? 1 : 0;   // warps per value (0: one warp takes all)
+    __syncthreads();
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        if (per ? warp / per != v : warp != 0) continue;
+        const int q = per ? warp % per : 0, np = per ? per : 1;
+        double s = 0.0;
+        for (int i = lane + 32 * q; i < count; i += 32 * np) s += (double)in[v * stride + i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) warp_sums[4 * v + q] = s;
+    }
+    __syncthreads();
+    if (warp == 0)
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+            out[v] = per == 4 ? (warp_sums[4 * v] + warp_sums[4 * v + 1]) + (warp_sums[4 * v + 2] + warp_sums[4 * v + 3])
+                              : warp_sums[4 * v];
+}
+
+// T: double (IML CG) or float (mixed). RPT: node rows per group of four threads (up
+// to 512 threads of 128 registers; with 1,024 threads of 64 the spilled values had to
+// be written back at every exchange's fence: 6.8 us an exchange).
+constexpr int NT = 512;
+template <int ND, class T, int RPT>
+__global__ void __launch_bounds__(NT, 1) k_pcg_persist(PersistArgs a)
+{
+    constexpr bool MIXED = sizeof(T) == 4;
+    constexpr int NV = ND * ND, NSYM = ND * (ND + 1) / 2;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ double warp_sums[8];
+    __shared__ double part_d[MIXED ? 1 : 2 * NT];                 // FP64 terms per thread
+    __shared__ float part_f[MIXED ? 2 * (NT / PARTS) * RPT : 1];  // mixed: r.r and r.z per node row
+    __shared__ double pq_d[MIXED ? NT : 1];
+    __shared__ PcgScal S;
+    __shared__ bool fine;
+    const int nt = blockDim.x, t = threadIdx.x, part = t & 3, lane = t & 31, group = t >> 2, groups = nt >> 2;
+    const int row0 = blockIdx.x * a.rows;
+    const T *val = static_cast<const T *>(a.val);
+    T *r_g = static_cast<T *>(a.r), *z_g = static_cast<T *>(a.z);
+    T *p_old = static_cast<T *>(a.p2), *p_new = static_cast<T *>(a.p);   // swapped in every iteration
+    if (t == 0) {
+        S = *a.sc;
+        fine = true;
+    }
+    __syncthreads();
+    if (S.done || S.reliable) return;   // the same in every CTA
+    Blocks<ND, T, RPT> M{reinterpret_cast<T *>(smem), reinterpret_cast<int *>(smem + (size_t)RPT * a.kc * NV * nt * sizeof(T)), nt,
+                         a.kc};
+    int row[RPT];
+    bool mine[RPT];     // this thread holds a degree of freedom of the row
+    int64_t slot0[RPT];
+    int width[RPT];
+    double x[RPT];
+    T r[RPT], p[RPT], d[RPT][MIXED ? ND : 1];
+#pragma unroll
+    for (int rp = 0; rp < RPT; ++rp) {
+        const int lr = group + rp * groups;
+        row[rp] = row0 + lr;
+        const bool on = lr < a.rows && row[rp] < a.nrows;
+        if (!on) row[rp] = 0;
+        slot0[rp] = a.sl_ptr[row[rp] >> 5] + (row[rp] & 31);
+        width[rp] = on ? a.sl_width[row[rp] >> 5] : 0;
+        mine[rp] = on && part < ND;
+        const int64_t i = (int64_t)row[rp] * ND + (part < ND ? part : 0);
+        x[rp] = mine[rp] ? a.x[i] : 0.0;
+        r[rp] = mine[rp] ? r_g[i] : (T)0;
+        p[rp] = mine[rp] ? p_new[i] : (T)0;
+        if constexpr (MIXED) {
+#pragma unroll
+            for (int j = 0; j < ND; ++j) {
+                const int hi = max(part, j), lo = min(part, j);
+                d[rp][j] = mine[rp] ? static_cast<const float *>(a.prec)[(int64_t)(lo * ND - lo * (lo - 1) / 2 + hi - lo) * a.planes + row[rp]]
+                                    : 0.f;
+            }
+        } else {
+            d[rp][0] = mine[rp] ? static_cast<const double *>(a.prec)[i] : 0.0;
+        }
+        for (int k = 0; k < a.kc; ++k) {
+            const int kk = k * PARTS + part;
+            const bool has = kk < width[rp];
+            const int64_t slot = slot0[rp] + 32 * (int64_t)kk;
+            *M.column(rp, k) = has ? a.col[slot] : row[rp];
+            const T *v = val + (slot - (row[rp] & 31)) * NV + (row[rp] & 31);
+#pragma unroll
+            for (int e = 0; e < NV; ++e) *M.value(rp, k, e) = has ? __ldcs(v + 32 * e) : (T)0;
+        }
+    }
+    double normb = sqrt(S.bnorm2);
+    if (normb == 0.0) normb = 1.0;
+    const double near = a.rtol * a.rtol * normb * normb * (1.0 + 1e-9);   // r.r above it: surely not converged
+    unsigned long long epoch = a.epoch;
+    bool first = true;   // p as it stands in memory; then p = z + beta p_old
+    T beta = 0;
+    for (int it = 0;; ++it) {
+        // q = K p (difference form in mixed solves), by four threads per row
+        T q[RPT];
+        double pq = 0.0;
+#pragma unroll
+        for (int rp = 0; rp < RPT; ++rp) {
+            T y[ND], pa[ND];
+#pragma unroll
+            for (int i = 0; i < ND; ++i) {
+                y[i] = 0;
+                pa[i] = MIXED ? __shfl_sync(0xffffffffu, p[rp], (lane & ~3) + i) : (T)0;
+            }
+            auto product = [&](int c, const T (&v)[NV]) {
+                T pc[ND];
+#pragma unroll
+                for (int j = 0; j < ND; ++j) {
+                    const int64_t i = (int64_t)c * ND + j;
+                    pc[j] = first ? p_new[i] : fma(beta, p_old[i], z_g[i]);
+                    if (MIXED && c != row[rp]) pc[j] -= pa[j];
+                }
+#pragma unroll
+                for (int i = 0; i < ND; ++i)
+#pragma unroll
+                    for (int j = 0; j < ND; ++j) y[i] += v[i * ND + j] * pc[j];
+            };
+#pragma unroll 4
+            for (int k = 0; k < a.kc; ++k) {
+                T v[NV];
+#pragma unroll
+                for (int e = 0; e < NV; ++e) v[e] = *M.value(rp, k, e);
+                product(*M.column(rp, k), v);
+            }
+            for (int k = a.kc; k < a.kmax; ++k) {
+                const int kk = k * PARTS + part;
+                if (kk >= width[rp]) break;
+                const int64_t slot = slot0[rp] + 32 * (int64_t)kk;
+                const T *vp = val + (slot - (row[rp] & 31)) * NV + (row[rp] & 31);
+                T v[NV];
+#pragma unroll
+                for (int e = 0; e < NV; ++e) v[e] = __ldg(vp + 32 * e);
+                product(__ldg(a.col + slot), v);
+            }
+            __syncwarp();
+            // parts 0, 1 and 2 end with components 0, 1 and 2: parts 0 and 1 take the
+            // first two from parts 2 and 3 and give them the third, then each pair
+            // completes one component per part (three additions instead of six)
+            if constexpr (ND == 3) {
+                const T y2 = __shfl_xor_sync(0xffffffffu, part < 2 ? y[2] : y[0], 2);
+                const T y1 = __shfl_xor_sync(0xffffffffu, y[1], 2);
+                const T h0 = (part < 2 ? y[0] : y[2]) + y2, h1 = y[1] + y1;   // parts 2, 3: h0 = component 2
+                const T give = __shfl_xor_sync(0xffffffffu, part == 0 ? h1 : h0, 1);
+                q[rp] = (part == 1 ? h1 : h0) + give;
+            } else {
+                const T give = __shfl_xor_sync(0xffffffffu, part & 1 ? y[0] : y[1], 1);
+                const T h = (part & 1 ? y[1] : y[0]) + give;
+                q[rp] = h + __shfl_xor_sync(0xffffffffu, h, 2);
+            }
+            if (mine[rp]) pq += (double)p[rp] * (double)q[rp];
+        }
+        double *terms = MIXED ? pq_d : part_d;
+        terms[t] = pq;
+        double one[1], s1[1];
+        cta_sum<1>(terms, nt, nt, one, warp_sums);
+        if (t < 32) {
+            const bool ok = exchange<1, false>(a.mail, epoch, one, s1);
+            const double alpha = S.rho / s1[0];
+            if (t == 0) {
+                fine = ok;
+                S.pq = s1[0];
+                if (!(s1[0] > 0.0) || !isfinite(s1[0])) S.done = 2;
+                else S.alpha = alpha;
+            }
+        }
+        ++epoch;
+        __syncthreads();
+        if (!fine || S.done) break;
+        // x, r, z and the sums r.r, r.z
+        const double alpha = S.alpha;
+        T z[RPT];
+        double rr = 0.0, rz = 0.0;
+#pragma unroll
+        for (int rp = 0; rp < RPT; ++rp) {
+            x[rp] += alpha * (double)p[rp];
+            if constexpr (MIXED) {
+                r[rp] = fmaf(-(float)alpha, q[rp], r[rp]);
+                if (!mine[rp]) r[rp] = 0.f;
+                float zz = 0.f;
+#pragma unroll
+                for (int j = 0; j < ND; ++j) zz = fmaf(d[rp][j], __shfl_sync(0xffffffffu, r[rp], (lane & ~3) + j), zz);
+                z[rp] = zz;
+                if (mine[rp]) z_g[(int64_t)row[rp] * ND + part] = zz;
+                float s0 = r[rp] * r[rp], s2 = r[rp] * zz;   // the node's sums in FP32
+                s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+                s2 += __shfl_xor_sync(0xffffffffu, s2, 1);
+                s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
+                s2 += __shfl_xor_sync(0xffffffffu, s2, 2);
+                if (part == 0) part_f[rp * groups + group] = s0;
+                if (part == 1) part_f[(RPT + rp) * groups + group] = s2;
+            } else {
+                r[rp] -= alpha * q[rp];
+                z[rp] = r[rp] * d[rp][0];
+                if (mine[rp]) {
+                    z_g[(int64_t)row[rp] * ND + part] = z[rp];
+                    rr += r[rp] * r[rp];
+                    rz += r[rp] * z[rp];
+                }
+            }
+        }
+        double two[2], s2[2];
+        if constexpr (MIXED) {
+            cta_sum<2>(part_f, RPT * groups, RPT * groups, two, warp_sums);
+        } else {
+            part_d[t] = rr;
+            part_d[nt + t] = rz;
+            cta_sum<2>(part_d, nt, nt, two, warp_sums);
+        }
+        if (t < 32) {
+            const bool ok = exchange<2, true>(a.mail, epoch, two, s2);
+            const double b = s2[1] / S.rho;
+            if (t == 0) {
+                fine = ok;
+                S.rnorm2 = s2[0];
+                S.iters += 1;
+                if (MIXED) {
+                    if (!isfinite(s2[0]) || !isfinite(s2[1])) S.done = 2;
+                    else if (s2[0] <= S.drop2 * S.rmax2 || s2[0] <= S.tol2 || !(s2[1] > 0.0) || S.iters >= a.maxit ||
+                             S.iters >= S.cycle_end)
+                        S.reliable = 1;
+                } else {
+                    if (!(s2[0] > near) && sqrt(s2[0]) / normb <= a.rtol) S.done = 1;
+                    else if (!isfinite(s2[1]) || !(s2[1] > 0.0)) S.done = 2;
+                    else if (S.iters >= a.maxit) S.done = 4;
+                }
+                if (!S.done && !S.reliable) {
+                    S.beta = b;
+                    S.rho_old = S.rho;
+                    S.rho = s2[1];
+                    S.zcoef = 1.0;
+                }
+            }
+        }
+        ++epoch;
+        __syncthreads();
+        // (a replacement continues from the p of this iteration)
+        if (!fine || S.done || S.reliable) break;
+        beta = (T)S.beta;
+        first = false;
+        T *swap = p_old;
+        p_old = p_new;
+        p_new = swap;
+#pragma unroll
+        for (int rp = 0; rp < RPT; ++rp) {
+            p[rp] = fma(beta, p[rp], z[rp]);
+            if (mine[rp]) p_new[(int64_t)row[rp] * ND + part] = p[rp];
+        }
+        if (it + 1 == BUDGET) break;
+    }
+#pragma unroll
+    for (int rp = 0; rp < RPT; ++rp)
+        if (mine[rp]) {
+            const int64_t i = (int64_t)row[rp] * ND + part;
+            a.x[i] = x[rp];
+            r_g[i] = r[rp];
+            static_cast<T *>(a.p)[i] = p[rp];
+        }
+    if (!fine && t == 0) atomicCAS(&a.sc->done, 0, WAIT_TIMEOUT);
+    if (fine && t == 0 && blockIdx.x == 0) *a.sc = S;
+}
+
+template <int ND, class T>
+const void *persist_fn(int rpt)
+{
+    switch (rpt) {
+    case 1: return (const void *)k_pcg_persist<ND, T, 1>;
+    case 2: return (const void *)k_pcg_persist<ND, T, 2>;
+    case 3: return (const void *)k_pcg_persist<ND, T, 3>;
+    default: return (const void *)k_pcg_persist<ND, T, 4>;
+    }
+}
+
+}  // namespace
+
+// Whether the systems of S run their iterations in one launch, and the launch's
+// shape: rows per CTA (a multiple of eight, so that the streamed blocks' loads keep
+// whole sectors), threads, blocks per thread in shared memory.
+bool persist_plan(const ogb_ctx *ctx, const SellMat &S, bool mixed, PersistPlan &P)
+{
+    if (!ctx->persist || ctx->prof || S.ninst > 1 || S.nact < 1) return false;
+    const int sms = num_sms();
+    if (sms > MAX_CTAS) return false;
+    // above 512 rows per SM (the size from which the multi-launch SpMV has one warp
+    // per slice and, in mixed solves, the half-stored operator) the launches' latency
+    // is a small part and the streaming kernels are faster
+    int64_t rows = std::max<int64_t>(8, ceil_div(ceil_div(S.nact, sms), 8) * 8);
+    if (rows > 512) return false;
+    P.rows = (int)rows;
+    P.grid = (int)ceil_div(S.nact, rows);
+    P.rpt = (int)ceil_div(rows, NT / PARTS);
+    P.nt = (int)ceil_div(ceil_div(rows, P.rpt) * PARTS, 32) * 32;
+    P.kmax = (int)ceil_div(S.max_width, PARTS);
+    const int64_t block = (int64_t)S.nd * S.nd * (mixed ? 4 : 8) + 4;
+    P.kc = (int)std::min<int64_t>(P.kmax, (SMEM_LIMIT - STATIC_SMEM) / (block * P.nt * P.rpt));
+    P.smem = (size_t)block * P.nt * P.rpt * P.kc;
+    return true;
+}
+
+int persist_run(ogb_mtrx *m, const PersistPlan &P, bool mixed, const void *val, double *x, void *r, void *p, void *z, void *p2, const void *prec,
+                double rtol, int maxit)
+{
+    ogb_ctx *ctx = m->ctx;
+    cudaStream_t s = ctx->stream;
+    const SellMat &S = m->sell;
+    const size_t boxes = (size_t)4 * P.grid * P.grid;
+    if (m->w_mail.n < 2 * boxes) {
+        OGB_CHECK(m->w_mail.alloc(2 * boxes));
+        OGB_CUDA(cudaMemsetAsync(m->w_mail.p, 0, m->w_mail.n * sizeof(double), s));   // epoch 0: no exchange's
+    }
+    const void *fn = mixed ? (S.nd == 3 ? persist_fn<3, float>(P.rpt) : persist_fn<2, float>(P.rpt))
+                           : (S.nd == 3 ? persist_fn<3, double>(P.rpt) : persist_fn<2, double>(P.rpt));
+    PersistArgs a{};
+    a.nrows = S.nact;
+    a.rows = P.rows;
+    a.kmax = P.kmax;
+    a.kc = P.kc;
+    a.sl_ptr = S.sl_ptr.p;
+    a.sl_width = S.sl_width.p;
+    a.col = S.col.p;
+    a.val = val;
+    a.x = x;
+    a.r = r;
+    a.p = p;
+    a.z = z;
+    a.p2 = p2;
+    a.prec = prec;
+    a.planes = (int64_t)S.nslices * 32;
+    a.mail = reinterpret_cast<Mail *>(m->w_mail.p);
+    a.epoch = m->mail_epoch + 1;
+    m->mail_epoch += 2 * BUDGET;   // epochs are never used twice
+    a.sc = m->w_scal.p;
+    a.rtol = rtol;
+    a.maxit = maxit;
+    OGB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT - STATIC_SMEM));
+    void *args[] = {&a};
+    const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(P.grid), dim3(P.nt), args, P.smem, s);
+    if (e != cudaSuccess) return cuda_fail(e, "cooperative launch of the CG iterations");
+    count_launch(ctx);
+    return OGB_OK;
+}
+
+}  // namespace ogb

@@ -1719,12 +1719,24 @@ int pcg64_core(ogb_mtrx *m, const Op &op, const double *val, const double *b, do
     PcgScal *sc = m->w_scal.p;
     double *r = m->w_r.p, *z = m->w_z.p, *p = m->w_p.p, *q = m->w_q.p, *dinv = m->w_dinv.p;
     OGB_CUDA(cudaMemsetAsync(sc, 0, sizeof(PcgScal), s));
-    OGB_CHECK((sell_autotune<double, double, double, false>(ctx, op, val, p, q, m->w_part.p, m->w_count.p, sc + 1)));
+    PersistPlan plan;
+    const bool persist = op.sell && persist_plan(ctx, *op.S, false, plan);
+    if (!persist)
+        OGB_CHECK((sell_autotune<double, double, double, false>(ctx, op, val, p, q, m->w_part.p, m->w_count.p, sc + 1)));
     OGB_CHECK((launch_prec_diag<double, double>(m, op, val, dinv, sc)));
     OGB_CHECK((apply_op<double, double, false>(ctx, op, val, x, q, nullptr, nullptr, nullptr)));
     k_pcg_init<double><<<g, NTHREADS, 0, s>>>(nch, b, q, dinv, r, z, p, m->w_part.p, m->w_count.p, sc, rtol);
     count_launch(ctx);
     OGB_CUDA(cudaGetLastError());
+    if (persist) {
+        for (;;) {
+            OGB_CHECK(read_scal(m, res));
+            if (res.done == DONE_WAIT_TIMEOUT)
+                return fail(OGB_E_CUDA, "CG iterations: the blocks did not all arrive within the wait limit");
+            if (res.done || res.iters >= maxit) return OGB_OK;
+            OGB_CHECK(persist_run(m, plan, false, val, x, r, p, z, q, dinv, rtol, maxit));
+        }
+    }
     auto batch = [&]() -> int {
         for (int k = 0; k < BATCH; ++k) {
             ctx->prof_sample = k == BATCH / 2 || !ctx->capture_events;   // time one mid-batch SpMV per replay
@@ -1968,7 +1980,12 @@ int pcg_mixed_core(ogb_mtrx *m, const Op &op, const double *v64, const float *v3
         }
     }
     m->last_half = half;
-    if (half) {
+    // small systems: the iterations between two replacements in one launch
+    PersistPlan plan;
+    const bool persist = F32 && sizeof(P) == 4 && bj && diff && !half && ctx->mixed_x64 && !ctx->mixed_sum32 &&
+                         persist_plan(ctx, *op.S, true, plan);
+    if (persist) {
+    } else if (half) {
         if constexpr (sizeof(P) == 4) {
             if (!ctx->half_form) {
                 if (diff) OGB_CHECK((half_autotune<P, true>(ctx, op, p, q, m->w_part.p, m->w_count.p, sc + 1)));
@@ -2033,7 +2050,7 @@ int pcg_mixed_core(ogb_mtrx *m, const Op &op, const double *v64, const float *v3
         return OGB_OK;
     };
     IterGraph graph;
-    if (ctx->use_graphs) OGB_CHECK(graph.capture(ctx, batch));
+    if (ctx->use_graphs && !persist) OGB_CHECK(graph.capture(ctx, batch));
     for (;;) {
         // FP64 residual of the current x64 (not sampled by the kernel timing, which
         // measures the FP32 operator of the iterations)
@@ -2095,9 +2112,11 @@ int pcg_mixed_core(ogb_mtrx *m, const Op &op, const double *v64, const float *v3
         // iterations on the FP32 operator until the next replacement is due
         for (int nb = 0;; ++nb) {
             OGB_CHECK(read_scal(m, res));
-            if (ctx->use_graphs && nb > 0) graph.harvest(ctx);
+            if (ctx->use_graphs && !persist && nb > 0) graph.harvest(ctx);
             if (res.done || res.reliable) break;
-            if (ctx->use_graphs) {
+            if (persist) {
+                OGB_CHECK(persist_run(m, plan, true, v32, x, r, p, z, q, binv, rtol, maxit));
+            } else if (ctx->use_graphs) {
                 OGB_CHECK(graph.launch(ctx));
                 count_launch(ctx, (bj && fuse ? 2 : 3) * BATCH + (F32 && !ctx->mixed_x64 ? 1 : 0));
             } else {
@@ -2107,7 +2126,7 @@ int pcg_mixed_core(ogb_mtrx *m, const Op &op, const double *v64, const float *v3
         longest = res.iters - iters > longest ? res.iters - iters : longest;
         iters = res.iters;
         if (res.done == DONE_WAIT_TIMEOUT)
-            return fail(OGB_E_CUDA, "fused block-Jacobi update: the blocks did not all arrive within the wait limit");
+            return fail(OGB_E_CUDA, "block-Jacobi CG iterations: the blocks did not all arrive within the wait limit");
         if (res.done == 3) { status = OGB_E_ZERODIAG; break; }
         if (res.done == 2) {   // FP32 recurrences broke down: finish in FP64
             *stalled = true;

@@ -508,3 +508,41 @@ def test_option_ranges_are_checked(native_lib):
     for opt, good in ((native_lib.OPT_HALF_FORM, 6), (native_lib.OPT_MIXED_X64, 3), (native_lib.OPT_BATCH_FORM, 2),
                       (native_lib.OPT_UPDATE_BLOCKS, 8), (native_lib.OPT_FUSED_UPDATE, 0), (native_lib.OPT_BATCH_X64, 1)):
         c.set_option(opt, good)
+
+
+@pytest.mark.parametrize("mesh,size", [("hex", (1, 1, 1)), ("hex", (6, 3, 3)), ("hex", (40, 8, 8)), ("hex", (60, 12, 12)),
+                                       ("hex", (70, 22, 18)), ("hex", (80, 23, 21)), ("hex", (100, 27, 25)), ("quad", 3),
+                                       ("quad", 60), ("quad", 190), ("tet", 7), ("tet", 24)])
+def test_one_launch_iterations(mesh, size, native_lib):
+    """CG iterations in one launch (systems of up to 512 node rows per SM) against
+    the per-iteration launches, which any option that chooses a form of them keeps:
+    one CTA and many, one to four node rows per thread, matrices that fit the shared
+    memory and matrices partly streamed, two and three DOFs per node. Both stop at
+    the same tolerance on the same system, so they differ by the tolerance times the
+    condition number at most (below 1e5 for these, 1e-12 and 1e-10); every form is
+    bitwise reproducible."""
+    from oofem_gb300 import meshgen as mg
+    m = mg.hex_cantilever(*size, jitter=0.2, seed=3) if mesh == "hex" else \
+        mg.quad_rve(size, seed=3) if mesh == "quad" else mg.tet_cube_linear(size, jitter=0.15, seed=3)
+    for prec, rtol, tol in ((native_lib.PREC_FP64, 1e-12, 1e-7), (native_lib.PREC_MIXED, 1e-10, 1e-6)):
+        out = []
+        for forced in (False, False, True):
+            c = native_lib.Context(0)
+            if forced:
+                c.set_option(native_lib.OPT_FUSED_UPDATE, 1)
+            model = native_lib.GpuModel(c, m)
+            A = native_lib.GpuCsrMtrx(c)
+            u, reac, info = model.linear_static(A, rtol=rtol, maxit=100000, precision=prec)
+            assert info.status == 0 and info.achieved <= rtol
+            out.append((u, reac, info.iterations, c.kernel_launches()))
+        a, b, f = out
+        assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1]) and a[2] == b[2]
+        assert rel(a[0], f[0]) < tol and rel(a[1], f[1]) < tol, (rel(a[0], f[0]), rel(a[1], f[1]))
+        assert a[3] < f[3] or f[2] < 8
+    # the iteration limit holds as before
+    _, _, info = model.linear_static(A, rtol=1e-30, maxit=5)
+    c = native_lib.Context(0)
+    model = native_lib.GpuModel(c, m)
+    A = native_lib.GpuCsrMtrx(c)
+    _, _, one = model.linear_static(A, rtol=1e-30, maxit=5)
+    assert one.iterations == info.iterations and one.status == info.status
