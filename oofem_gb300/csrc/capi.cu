@@ -773,6 +773,7 @@ int ogb_model_create(ogb_ctx *ctx, int etype, int nnodes, const double *coords, 
     md->nmat = nmat;
     md->thickness = thickness;
     md->nonlinear = nonlinear;
+    for (int i = 0; i < nmat; ++i) md->has_idm1 |= (int)mats[8 * i] == OGB_MAT_IDM1;
     // a1: equation numbering (engngm.C:469-530, masterdof.C:105-120)
     md->h_eq.resize((size_t)nnodes * ndofpn);
     int neq = 0, npeq = 0;

@@ -52,16 +52,17 @@ __device__ void hex_grad(const R (&x)[8][3], int gp, R (&g)[8][3], R &dV)
     R c01 = J[1][0] * J[2][2] - J[1][2] * J[2][0];
     R c02 = J[1][0] * J[2][1] - J[1][1] * J[2][0];
     R det = J[0][0] * c00 - J[0][1] * c01 + J[0][2] * c02;
+    const R rd = R(1) / det;   // (nine divisions were a third of the FP64 work of a point)
     R Ji[3][3];
-    Ji[0][0] = c00 / det;
-    Ji[0][1] = (J[0][2] * J[2][1] - J[0][1] * J[2][2]) / det;
-    Ji[0][2] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) / det;
-    Ji[1][0] = -c01 / det;
-    Ji[1][1] = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) / det;
-    Ji[1][2] = (J[0][2] * J[1][0] - J[0][0] * J[1][2]) / det;
-    Ji[2][0] = c02 / det;
-    Ji[2][1] = (J[0][1] * J[2][0] - J[0][0] * J[2][1]) / det;
-    Ji[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) / det;
+    Ji[0][0] = c00 * rd;
+    Ji[0][1] = (J[0][2] * J[2][1] - J[0][1] * J[2][2]) * rd;
+    Ji[0][2] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) * rd;
+    Ji[1][0] = -c01 * rd;
+    Ji[1][1] = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) * rd;
+    Ji[1][2] = (J[0][2] * J[1][0] - J[0][0] * J[1][2]) * rd;
+    Ji[2][0] = c02 * rd;
+    Ji[2][1] = (J[0][1] * J[2][0] - J[0][0] * J[2][1]) * rd;
+    Ji[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * rd;
 #pragma unroll
     for (int a = 0; a < 8; ++a)
 #pragma unroll
@@ -84,7 +85,8 @@ __device__ void quad_grad_at(const R (&x)[4][2], R ksi, R eta, R (&g)[4][2], R &
         j10 += dn1[i] * x[i][0]; j11 += dn1[i] * x[i][1];
     }
     det = j00 * j11 - j01 * j10;
-    const R i00 = j11 / det, i01 = -j01 / det, i10 = -j10 / det, i11 = j00 / det;
+    const R rd = R(1) / det;
+    const R i00 = j11 * rd, i01 = -j01 * rd, i10 = -j10 * rd, i11 = j00 * rd;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         g[i][0] = i00 * dn0[i] + i01 * dn1[i];
@@ -177,46 +179,56 @@ __device__ __forceinline__ double norm_dev(const double (&s)[6])
 // MisesMat::performPlasticityReturn 3-D branch (misesmat.C:181-263), htype 0, no damage.
 // State (24 doubles): [0..5] eps_p, [6] kappa (committed); [8..13] eps_p, [14] kappa (temp);
 // [15..20] trial deviatoric stress, [21] trial volumetric stress.
-__device__ void mises_stress(const double *mat, const double (&eps)[6], double *st, double (&sig)[6])
+// G and 3 K come from the elastic matrix of the material (D_44 and D_11 + 2 D_12);
+// the norm's root and the return are taken only past the yield surface (compared by
+// squares first), with one division for dKappa / |s|: FP64 divisions and roots are
+// ten and more instructions each on the narrow FP64 pipe.
+__device__ __forceinline__ void mises_stress(const double *mat, const double *Del, const double (&eps)[6], double *st,
+                                             double (&sig)[6], bool write)
 {
-    double E = mat[1], nu = mat[2], sig0 = mat[3], H = mat[4];
-    double G = E / (2.0 * (1. + nu));
-    double K = E / (3.0 * (1. - 2. * nu));
-    double pl[6];
+    const double sig0 = mat[3], H = mat[4], G = __ldg(Del + 21), K3 = __ldg(Del) + 2.0 * __ldg(Del + 1);
+    double pl[6], el[6];
 #pragma unroll
-    for (int i = 0; i < 6; ++i) pl[i] = st[i];
+    for (int i = 0; i < 6; ++i) {
+        pl[i] = st[i];
+        el[i] = eps[i] - pl[i];
+    }
     double kappa = st[6];
-    double el[6];
+    const double mean = (el[0] + el[1] + el[2]) * (1.0 / 3.0), g2 = 2.0 * G;
+    double s[6] = {g2 * (el[0] - mean), g2 * (el[1] - mean), g2 * (el[2] - mean), G * el[3], G * el[4], G * el[5]};
+    const double svol = K3 * mean;
+    if (write) {
 #pragma unroll
-    for (int i = 0; i < 6; ++i) el[i] = eps[i] - pl[i];
-    double mean = (el[0] + el[1] + el[2]) / 3.0;
-    double s[6] = {2. * G * (el[0] - mean), 2. * G * (el[1] - mean), 2. * G * (el[2] - mean),
-                   G * el[3], G * el[4], G * el[5]};
-    double svol = 3 * K * mean;
+        for (int i = 0; i < 6; ++i) st[15 + i] = s[i];
+        st[21] = svol;
+    }
+    const double ss = s[0] * s[0] + s[1] * s[1] + s[2] * s[2] + 2.0 * (s[3] * s[3] + s[4] * s[4] + s[5] * s[5]);
+    const double sy = sig0 + H * kappa;
+    if (!(sy > 0.0) || 1.5 * ss > sy * sy * (1.0 - 1e-12)) {
+        const double trialS = sqrt(ss);
+        const double yieldValue = sqrt(3. / 2.) * trialS - sy;
+        if (yieldValue > 0.) {
+            const double q = yieldValue / ((H + 3. * G) * trialS);   // dKappa / |s|
+            kappa += q * trialS;
+            const double f = sqrt(3. / 2.) * q;
+            pl[0] += f * s[0];
+            pl[1] += f * s[1];
+            pl[2] += f * s[2];
+            pl[3] += 2.0 * f * s[3];
+            pl[4] += 2.0 * f * s[4];
+            pl[5] += 2.0 * f * s[5];
+            const double sc = 1. - sqrt(6.) * G * q;
 #pragma unroll
-    for (int i = 0; i < 6; ++i) st[15 + i] = s[i];
-    st[21] = svol;
-    double trialS = norm_dev(s);
-    double yieldValue = sqrt(3. / 2.) * trialS - (sig0 + H * kappa);
-    if (yieldValue > 0.) {
-        double dKappa = yieldValue / (H + 3. * G);
-        kappa += dKappa;
-        double f = sqrt(3. / 2.) * dKappa / trialS;
-        pl[0] += f * (1. / (2. * 0.5) * s[0]);
-        pl[1] += f * (1. / (2. * 0.5) * s[1]);
-        pl[2] += f * (1. / (2. * 0.5) * s[2]);
-        pl[3] += f * (1. / 0.5 * s[3]);
-        pl[4] += f * (1. / 0.5 * s[4]);
-        pl[5] += f * (1. / 0.5 * s[5]);
-        double sc = 1. - sqrt(6.) * G * dKappa / trialS;
-#pragma unroll
-        for (int i = 0; i < 6; ++i) s[i] *= sc;
+            for (int i = 0; i < 6; ++i) s[i] *= sc;
+        }
     }
     sig[0] = s[0] + svol; sig[1] = s[1] + svol; sig[2] = s[2] + svol;
     sig[3] = s[3]; sig[4] = s[4]; sig[5] = s[5];
+    if (write) {
 #pragma unroll
-    for (int i = 0; i < 6; ++i) st[8 + i] = pl[i];
-    st[14] = kappa;
+        for (int i = 0; i < 6; ++i) st[8 + i] = pl[i];
+        st[14] = kappa;
+    }
 }
 
 // MisesMat::give3dMaterialStiffnessMatrix (misesmat.C:496-535), TangentStiffness, omega 0.
@@ -434,6 +446,370 @@ __device__ void idm1_stress(const double *mat, const double (&eps)[6], double *s
     st[2] = le;
 }
 
+// ------------------------------------------------------------------ LSpace by its tensor structure
+// Eight lanes share a hexahedron: lane l = (bu, bv, bw) is Gauss point l of the
+// reference's order and holds the node on the same side of each axis (the point
+// nearest to it). A derivative along u at the point is the difference of the two
+// faces along u, interpolated along v and w; with the nearer node's weight taken out,
+// a step of interpolation is one multiply-add, x_near + HEX_FAR x_far, and the weight,
+// ((1 + g) / 2)^2 / 2 per derivative, cancels in grad u = (du/dxi)(dx/dxi)^-1 and
+// comes back as its cube in the forces. The transposed steps take the weighted
+// stresses to the nodes. Per point that is 27 FP64 instructions for dx/dxi and
+// du/dxi together and 36 for the forces, where full gradients of eight nodes at every point
+// took 144, 72 and 72, and the exchanges by shuffle cost next to nothing beside the
+// FP64 pipe, which bounds these kernels (two lanes per clock on an SM).
+constexpr double HEX_G = 0.577350269189626;   // as c_gp2
+constexpr double HEX_FAR = (1.0 - HEX_G) / (1.0 + HEX_G);
+constexpr double HEX_W = 0.125 * (1.0 + HEX_G) * (1.0 + HEX_G);
+
+// Node of lane l's octant (fei3dhexalin.C node order).
+__device__ __forceinline__ int hex_node(int l)
+{
+    const int bu = (l >> 2) & 1, bv = (l >> 1) & 1, bw = l & 1;
+    return (bw ? 0 : 4) + (bu ? 3 - bv : bv);
+}
+
+__device__ __forceinline__ double lane_xor(double v, int m) { return __shfl_xor_sync(0xffffffffu, v, m); }
+
+// d[k] = dX/dxi_k / HEX_W at this lane's point from the nodes' values X (one per lane).
+__device__ __forceinline__ void hex_derivatives(double X, int l, double (&d)[3])
+{
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int ax = 4 >> k, m1 = k == 0 ? 2 : 4, m2 = k == 2 ? 2 : 1;   // the axis' lane bit, the other two
+        const double o = lane_xor(X, ax);
+        double v = (l & ax) ? X - o : o - X;
+        v = fma(HEX_FAR, lane_xor(v, m1), v);
+        d[k] = fma(HEX_FAR, lane_xor(v, m2), v);
+    }
+}
+
+// The derivatives of two fields X and U: the difference along an axis is the same in
+// both lanes of a pair, so one lane takes X through it and the other U.
+__device__ __forceinline__ void hex_derivatives2(double X, double U, int l, double (&dX)[3], double (&dU)[3])
+{
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int ax = 4 >> k, m1 = k == 0 ? 2 : 4, m2 = k == 2 ? 2 : 1;
+        const bool hi = l & ax;
+        const double o = lane_xor(hi ? X : U, ax);   // the low lane gets the high X, the high lane the low U
+        double v = hi ? U - o : o - X;
+        v = fma(HEX_FAR, lane_xor(v, m1), v);
+        v = fma(HEX_FAR, lane_xor(v, m2), v);
+        const double w = lane_xor(v, ax);
+        dX[k] = hi ? w : v;
+        dU[k] = hi ? v : w;
+    }
+}
+
+// Transposed: value at this lane's node of sum over points of dN/dxi_k P_k / HEX_W.
+__device__ __forceinline__ double hex_to_node(const double (&P)[3], int l)
+{
+    double f = 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int ax = 4 >> k, m1 = k == 0 ? 2 : 4, m2 = k == 2 ? 2 : 1;
+        double v = P[k] + lane_xor(P[k], ax);
+        v = fma(HEX_FAR, lane_xor(v, m1), v);
+        v = fma(HEX_FAR, lane_xor(v, m2), v);
+        f += (l & ax) ? v : -v;
+    }
+    return f;
+}
+
+// Cofactors C of J (C = det J^-1) and the determinant.
+__device__ __forceinline__ double cofactors(const double (&J)[3][3], double (&C)[3][3])
+{
+    C[0][0] = J[1][1] * J[2][2] - J[1][2] * J[2][1];
+    C[0][1] = J[0][2] * J[2][1] - J[0][1] * J[2][2];
+    C[0][2] = J[0][1] * J[1][2] - J[0][2] * J[1][1];
+    C[1][0] = J[1][2] * J[2][0] - J[1][0] * J[2][2];
+    C[1][1] = J[0][0] * J[2][2] - J[0][2] * J[2][0];
+    C[1][2] = J[0][2] * J[1][0] - J[0][0] * J[1][2];
+    C[2][0] = J[1][0] * J[2][1] - J[1][1] * J[2][0];
+    C[2][1] = J[0][1] * J[2][0] - J[0][0] * J[2][1];
+    C[2][2] = J[0][0] * J[1][1] - J[0][1] * J[1][0];
+    return J[0][0] * C[0][0] + J[0][1] * C[1][0] + J[0][2] * C[2][0];
+}
+
+// Internal forces of LSpace elements (see k_elem_internal_forces), a thread per Gauss
+// point. Models without IDM1 have a form of their own: the damage update's registers
+// (166 a thread) would leave eight warps on an SM, too few to keep the FP64 pipe fed.
+// Measured (GB300, 101 x 37 x 37 hexes, MisesMat): 1,238 -> 540 us;
+// elastic, 290 x 58 x 58: 7.41 -> 2.85 ms.
+template <bool DAMAGE>
+__global__ void __launch_bounds__(NTHREADS, DAMAGE ? 1 : 2) k_hex_internal_forces(
+    int nelem, const double *__restrict__ coords, const int *__restrict__ conn, const int *__restrict__ emat,
+    const double *__restrict__ mats, const double *__restrict__ Dmat, const double *__restrict__ u_node,
+    double *__restrict__ state, double *__restrict__ gp_stress, double *__restrict__ gp_strain, double *__restrict__ fe)
+{
+    const int l = threadIdx.x & 7;
+    const int64_t ee = ((int64_t)blockIdx.x * NTHREADS + threadIdx.x) >> 3;
+    const bool on = ee < nelem;
+    const int e = on ? (int)ee : nelem - 1;   // lanes past the end help with the shuffles
+    const int a = hex_node(l), node = __ldg(conn + (size_t)e * 8 + a);
+    double J[3][3], dU[3][3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        hex_derivatives2(__ldg(coords + (size_t)node * 3 + i), __ldg(u_node + (size_t)node * 3 + i), l, J[i], dU[i]);
+    double C[3][3];
+    const double det = cofactors(J, C);
+    const double rd = 1.0 / det;
+    // grad u = dU J^-1 = dU C / det
+    double H[3][3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) H[i][j] = dU[i][0] * C[0][j] + dU[i][1] * C[1][j] + dU[i][2] * C[2][j];
+    const double eps[6] = {H[0][0] * rd, H[1][1] * rd, H[2][2] * rd, (H[1][2] + H[2][1]) * rd, (H[0][2] + H[2][0]) * rd,
+                           (H[0][1] + H[1][0]) * rd};
+    const int m = __ldg(emat + e);
+    const double *mat = mats + 8 * m, *Del = Dmat + 36 * m;
+    const int kind = (int)mat[0];
+    const size_t pt = (size_t)e * 8 + l;
+    double *st = state ? state + pt * NSTATE : nullptr;
+    double sig[6];
+    if (kind == OGB_MAT_MISES && st) {
+        mises_stress(mat, Del, eps, st, sig, on);
+    } else if (DAMAGE && kind == OGB_MAT_IDM1 && st) {
+        if constexpr (DAMAGE) {
+            double x[8][3], own[NSTATE];
+            gather_xe<OGB_LSPACE>(coords, conn, e, x);
+            for (int k = 0; k < 3; ++k) own[k] = st[k];
+            idm1_stress<8>(mat, eps, own, x, Del, sig);
+            if (on) {
+                st[2] = own[2];
+                st[8] = own[8];
+                st[9] = own[9];
+            }
+        }
+    } else {
+        // isotropic D: lambda tr(eps) 1 + 2 mu eps
+        const double lam = __ldg(Del + 1), mu2 = __ldg(Del) - lam, t = lam * (eps[0] + eps[1] + eps[2]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            sig[k] = fma(mu2, eps[k], t);
+            sig[3 + k] = __ldg(Del + 21) * eps[3 + k];
+        }
+    }
+    if (gp_stress && on) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            gp_stress[pt * 6 + k] = sig[k];
+            gp_strain[pt * 6 + k] = eps[k];
+        }
+    }
+    // P_ik = |det| sum_j sigma_ij J^-1_kj = sign(det) sum_j sigma_ij C_kj
+    const double sg = det < 0.0 ? -1.0 : 1.0;
+    const double S[3][3] = {{sig[0], sig[5], sig[4]}, {sig[5], sig[1], sig[3]}, {sig[4], sig[3], sig[2]}};
+    const double w = sg * (HEX_W * HEX_W * HEX_W);
+    double *out = fe + ((size_t)e * 8 + a) * 3;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        double P[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) P[k] = w * (S[i][0] * C[k][0] + S[i][1] * C[k][1] + S[i][2] * C[k][2]);
+        const double f = hex_to_node(P, l);
+        if (on) out[i] = f;
+    }
+}
+
+// Element stiffness of LSpace (layout of k_elem_stiffness): every D here is
+// lambda 1(x)1 + 2 mu I + c s(x)s, elastic (c = 0), damaged (lambda, mu scaled) or
+// MisesMat's consistent tangent (misesmat.C:496-535: factor2 I_dev moves lambda and
+// mu, factor1 is c, s the trial deviator), so with g_a the gradient of node a and
+// h_a = s g_a
+//   K_ab = sum_gp dV [lambda g_a g_b^T + mu g_b g_a^T + mu (g_a.g_b) 1 + c h_a h_b^T],
+// and K_ba = K_ab^T: of the 64 node pairs 36 are computed. Phase 1, a thread per Gauss
+// point: gradients and h of the eight nodes to shared memory. Phase 2, a thread per
+// node a: the pairs (a, a + 0..3 mod 8); the pair (a, a + 4) is shared by its two
+// threads, four Gauss points each. FP64-bound: 30 multiply-adds per pair and point
+// (9 when D is one elastic matrix: PLASTIC false sums only A_ab = dV g_a g_b^T) against
+// 43 for the dense D B of all 64 pairs.
+// Measured (GB300): MisesMat, 75 x 31 x 31 hexes 3.21 -> 1.61 ms; elastic,
+// 290 x 58 x 58: 16.4 -> 9.3 ms.
+template <bool PLASTIC>
+__global__ void __launch_bounds__(NTHREADS) k_hex_stiffness(
+    int nelem, const double *__restrict__ coords, const int *__restrict__ conn, const int *__restrict__ emat,
+    const double *__restrict__ mats, const double *__restrict__ Dmat, const double *__restrict__ state,
+    double *__restrict__ ke)
+{
+    constexpr int EPB = NTHREADS / 8, GP = 25;   // 24 gradient components of a point and a pad
+    extern __shared__ double smem[];
+    double *s_g = smem, *s_w = smem + EPB * 8 * GP, *s_h = s_w + EPB * 8 * (PLASTIC ? 3 : 1);
+    const int le = threadIdx.x >> 3, l = threadIdx.x & 7, e0 = blockIdx.x * EPB;
+    const bool on = e0 + le < nelem;
+    const int e = on ? e0 + le : nelem - 1;
+    const int m = __ldg(emat + e);
+    const double *Del = Dmat + 36 * m;
+    bool bent = false;   // the thread's point has c != 0
+    {
+        const int node = __ldg(conn + (size_t)e * 8 + hex_node(l));
+        double J[3][3], C[3][3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) hex_derivatives(__ldg(coords + (size_t)node * 3 + i), l, J[i]);
+        const double det = cofactors(J, C);
+        const double rd = 1.0 / (HEX_W * det);
+        const double dV = (HEX_W * HEX_W * HEX_W) * fabs(det);
+        double *g = s_g + (size_t)(le * 8 + l) * GP;
+        constexpr double NEAR = 0.5 * (1.0 + HEX_G), FAR = 0.5 * (1.0 - HEX_G);
+        double S[6] = {0, 0, 0, 0, 0, 0}, lam = __ldg(Del + 1), mu = __ldg(Del + 21), c = 0.0;
+        if constexpr (PLASTIC) {
+            const double *mat = mats + 8 * m, *st = state + ((size_t)e * 8 + l) * NSTATE;
+            const int kind = (int)mat[0];
+            if (kind == OGB_MAT_MISES) {
+                const double dKappa = st[14] - st[6];
+                if (dKappa > 0.0) {
+#pragma unroll
+                    for (int i = 0; i < 6; ++i) S[i] = st[15 + i];
+                    const double G = mu, H = mat[4], trialS = norm_dev(S);
+                    const double factor = -2. * sqrt(6.) * G * G / trialS;
+                    c = factor * (mat[3] + H * st[6]) / ((H + 3. * G) * trialS * trialS);
+                    const double f2 = factor * dKappa;
+                    mu += 0.5 * f2;
+                    lam -= f2 * (1.0 / 3.0);
+                    bent = true;
+                }
+            } else if (kind == OGB_MAT_IDM1) {
+                const double om = st[9] < 0.999999 ? st[9] : 0.999999;
+                lam *= 1.0 - om;
+                mu *= 1.0 - om;
+            }
+            double *w = s_w + (le * 8 + l) * 3;
+            w[0] = lam * dV;
+            w[1] = mu * dV;
+            w[2] = c * dV;
+        } else {
+            s_w[le * 8 + l] = dV;
+        }
+        const int bu = (l >> 2) & 1, bv = (l >> 1) & 1, bw = l & 1;
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) C[i][k] *= rd;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {   // node of octant q: signs su, sv, sw
+            const int qu = (q >> 2) & 1, qv = (q >> 1) & 1, qw = q & 1, a = hex_node(q);
+            const double nu = qu == bu ? NEAR : FAR, nv = qv == bv ? NEAR : FAR, nw = qw == bw ? NEAR : FAR;
+            const double du = (qu ? 0.5 : -0.5) * nv * nw, dv = (qv ? 0.5 : -0.5) * nu * nw, dw = (qw ? 0.5 : -0.5) * nu * nv;
+            double ga[3];
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                ga[j] = du * C[0][j] + dv * C[1][j] + dw * C[2][j];
+                g[a * 3 + j] = ga[j];
+            }
+            if constexpr (PLASTIC) {
+                double *h = s_h + (size_t)(le * 8 + l) * GP + a * 3;
+                if (bent) {
+                    h[0] = S[0] * ga[0] + S[5] * ga[1] + S[4] * ga[2];
+                    h[1] = S[5] * ga[0] + S[1] * ga[1] + S[3] * ga[2];
+                    h[2] = S[4] * ga[0] + S[3] * ga[1] + S[2] * ga[2];
+                } else {
+                    h[0] = h[1] = h[2] = 0.0;
+                }
+            }
+        }
+    }
+    // a warp reads only its own four elements' points
+    __syncwarp();
+    const unsigned any_bent = __ballot_sync(0xffffffffu, bent);
+    const int a = l;
+    constexpr int NB = 5;   // pairs of a thread; the last with half the points
+    double A[NB][9], tr[NB];
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
+        tr[k] = 0.0;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) A[k][i] = 0.0;
+    }
+#pragma unroll 1
+    for (int step = 0; step < 8; ++step) {
+        const int gp = (step + (a & 4)) & 7;   // threads a and a + 4 start half the points apart
+        const double *g = s_g + (size_t)(le * 8 + gp) * GP;
+        const double ga[3] = {g[a * 3], g[a * 3 + 1], g[a * 3 + 2]};
+        if constexpr (PLASTIC) {
+            const double *w = s_w + (le * 8 + gp) * 3, *h = s_h + (size_t)(le * 8 + gp) * GP;
+            const double la[3] = {w[0] * ga[0], w[0] * ga[1], w[0] * ga[2]};
+            const double ma[3] = {w[1] * ga[0], w[1] * ga[1], w[1] * ga[2]};
+            const bool ps = any_bent != 0;   // an elastic warp leaves the last term out
+            double ha[3] = {0.0, 0.0, 0.0};
+            if (ps) {
+#pragma unroll
+                for (int i = 0; i < 3; ++i) ha[i] = w[2] * h[a * 3 + i];
+            }
+#pragma unroll
+            for (int k = 0; k < NB; ++k) {
+                if (k == NB - 1 && step >= 4) break;
+                const int b = (a + k) & 7;
+                const double gb[3] = {g[b * 3], g[b * 3 + 1], g[b * 3 + 2]};
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    tr[k] = fma(ma[i], gb[i], tr[k]);
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) A[k][3 * i + j] = fma(ma[j], gb[i], fma(la[i], gb[j], A[k][3 * i + j]));
+                }
+                if (ps) {
+                    const double hb[3] = {h[b * 3], h[b * 3 + 1], h[b * 3 + 2]};
+#pragma unroll
+                    for (int i = 0; i < 3; ++i)
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) A[k][3 * i + j] = fma(ha[i], hb[j], A[k][3 * i + j]);
+                }
+            }
+        } else {
+            const double dv = s_w[le * 8 + gp];
+            const double la[3] = {dv * ga[0], dv * ga[1], dv * ga[2]};
+#pragma unroll
+            for (int k = 0; k < NB; ++k) {
+                if (k == NB - 1 && step >= 4) break;
+                const int b = (a + k) & 7;
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) A[k][3 * i + j] = fma(la[i], g[b * 3 + j], A[k][3 * i + j]);
+            }
+        }
+    }
+    // the shared pair: thread a < 4 adds what thread a + 4 has (that is pair (a + 4, a): transposed)
+    tr[NB - 1] += lane_xor(tr[NB - 1], 4);
+    {
+        double o[9];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) o[i] = lane_xor(A[NB - 1][i], 4);
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) A[NB - 1][3 * i + j] += o[3 * j + i];
+    }
+    if (!on) return;
+    const double lam = __ldg(Del + 1), mu = __ldg(Del + 21);
+    double *out = ke + (size_t)e * 64 * 9;
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
+        if (k == NB - 1 && a >= 4) break;
+        const int b = (a + k) & 7;
+        double K[9];
+        if constexpr (PLASTIC) {
+#pragma unroll
+            for (int i = 0; i < 9; ++i) K[i] = A[k][i] + (i % 4 == 0 ? tr[k] : 0.0);
+        } else {
+            const double mtr = mu * (A[k][0] + A[k][4] + A[k][8]);
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) K[3 * i + j] = lam * A[k][3 * i + j] + mu * A[k][3 * j + i] + (i == j ? mtr : 0.0);
+        }
+        double *ab = out + (a * 8 + b) * 9, *ba = out + (b * 8 + a) * 9;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) ab[i] = K[i];
+        if (k > 0)
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) ba[3 * j + i] = K[3 * i + j];
+    }
+}
+
 // ------------------------------------------------------------------ K1 stiffness
 // Ke layout: ke[e][a][b][i][j] (ND x ND node blocks, row-major).
 template <int ET, bool PER_GP_D>
@@ -500,46 +876,6 @@ __global__ void __launch_bounds__(NTHREADS) k_elem_stiffness(
 
     const int le = threadIdx.x / NPE, a = threadIdx.x % NPE, e = e0 + le;
     if (e >= nelem) return;
-    if constexpr (ET == OGB_LSPACE && !PER_GP_D) {
-        // Isotropic D (D = 2G I_dev + K 1(x)1, isolinearelasticmaterial.C:80-88): with
-        // lambda = D_12 and mu = D_44,
-        //   K_ab^ij = sum_gp dV [lambda g_a^i g_b^j + mu g_a^j g_b^i + mu delta_ij g_a.g_b]
-        // = lambda A_ab^ij + mu A_ab^ji + mu delta_ij tr A_ab,  A_ab^ij = sum_gp dV g_a^i g_b^j,
-        // the same B^T D B dV sum in a third of the FP64 operations of the dense product.
-        const double *Dm = Dmat + 36 * __ldg(emat + e);
-        const double lam = __ldg(Dm + 1), mu = __ldg(Dm + 21);
-        double A[NPE][3][3];
-#pragma unroll
-        for (int b = 0; b < NPE; ++b)
-#pragma unroll
-            for (int i = 0; i < 3; ++i)
-#pragma unroll
-                for (int j = 0; j < 3; ++j) A[b][i][j] = 0.0;
-#pragma unroll 1
-        for (int gp = 0; gp < NGP; ++gp) {
-            const double dv = s_dv[le][gp];
-            const double ga[3] = {dv * s_g[le][gp][a][0], dv * s_g[le][gp][a][1], dv * s_g[le][gp][a][2]};
-#pragma unroll
-            for (int b = 0; b < NPE; ++b) {
-                const double h[3] = {s_g[le][gp][b][0], s_g[le][gp][b][1], s_g[le][gp][b][2]};
-#pragma unroll
-                for (int i = 0; i < 3; ++i)
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) A[b][i][j] = fma(ga[i], h[j], A[b][i][j]);
-            }
-        }
-        double *out = ke + (((size_t)e * NPE + a) * NPE) * 9;
-#pragma unroll
-        for (int b = 0; b < NPE; ++b) {
-            const double mtr = mu * (A[b][0][0] + A[b][1][1] + A[b][2][2]);
-#pragma unroll
-            for (int i = 0; i < 3; ++i)
-#pragma unroll
-                for (int j = 0; j < 3; ++j)
-                    out[(b * 3 + i) * 3 + j] = lam * A[b][i][j] + mu * A[b][j][i] + (i == j ? mtr : 0.0);
-        }
-        return;
-    }
     double D[NS][NS];
     if constexpr (!PER_GP_D) {
         const double *Dm = Dmat + 36 * __ldg(emat + e);
@@ -682,7 +1018,7 @@ __global__ void __launch_bounds__(NTHREADS) k_elem_internal_forces(
                 double e6[6], s6[6];
 #pragma unroll
                 for (int k = 0; k < 6; ++k) e6[k] = eps[k];
-                mises_stress(mat, e6, st, s6);
+                mises_stress(mat, Del, e6, st, s6, true);
 #pragma unroll
                 for (int k = 0; k < 6; ++k) sig[k] = s6[k];
             } else if (kind == OGB_MAT_IDM1 && st) {
@@ -783,6 +1119,16 @@ template <int ET, bool PERGP>
 static int run_stiffness(ogb_model *md)
 {
     ogb_ctx *ctx = md->ctx;
+    if constexpr (ET == OGB_LSPACE) {
+        constexpr size_t hs = sizeof(double) * (NTHREADS * (PERGP ? 25 + 3 + 25 : 25 + 1));
+        static bool hex_set[64] = {};
+        OGB_CUDA(set_smem_limit_once((const void *)k_hex_stiffness<PERGP>, (int)hs, hex_set));
+        k_hex_stiffness<PERGP><<<(unsigned)ceil_div((int64_t)md->nelem * 8, NTHREADS), NTHREADS, hs, ctx->stream>>>(
+            md->nelem, md->coords.p, md->conn.p, md->emat.p, md->mats.p, md->Dmat.p, md->state.p, md->ke.p);
+        count_launch(ctx);
+        OGB_CUDA(cudaGetLastError());
+        return OGB_OK;
+    } else {
     constexpr size_t smem = stiff_smem<ET>(PERGP);
     static bool attr_set[64] = {};
     OGB_CUDA(set_smem_limit_once((const void *)k_elem_stiffness<ET, PERGP>, (int)smem, attr_set));
@@ -793,12 +1139,22 @@ static int run_stiffness(ogb_model *md)
     count_launch(ctx);
     OGB_CUDA(cudaGetLastError());
     return OGB_OK;
+    }
 }
 
 template <int ET>
 static int run_forces(ogb_model *md, const double *u_node)
 {
     ogb_ctx *ctx = md->ctx;
+    if constexpr (ET == OGB_LSPACE) {
+        auto fn = md->has_idm1 ? k_hex_internal_forces<true> : k_hex_internal_forces<false>;
+        fn<<<(unsigned)ceil_div((int64_t)md->nelem * 8, NTHREADS), NTHREADS, 0, ctx->stream>>>(
+            md->nelem, md->coords.p, md->conn.p, md->emat.p, md->mats.p, md->Dmat.p, u_node,
+            md->nonlinear ? md->state.p : nullptr, md->gp_stress.p, md->gp_strain.p, md->fe.p);
+        count_launch(ctx);
+        OGB_CUDA(cudaGetLastError());
+        return OGB_OK;
+    } else {
     constexpr size_t smem = force_smem<ET>();
     static bool attr_set[64] = {};
     OGB_CUDA(set_smem_limit_once((const void *)k_elem_internal_forces<ET>, (int)smem, attr_set));
@@ -810,6 +1166,7 @@ static int run_forces(ogb_model *md, const double *u_node)
     count_launch(ctx);
     OGB_CUDA(cudaGetLastError());
     return OGB_OK;
+    }
 }
 
 // ------------------------------------------------------------------ K1 on tensor cores

@@ -344,6 +344,7 @@ struct ogb_model {
     ogb::DBuf<double> v_unode, v_fnode, v_bcval, v_load, v_b, v_x, v_reac;
     ogb_mtrx *bound = nullptr;
     bool nonlinear = false;
+    bool has_idm1 = false;       // some material is IDM1
     std::vector<int> inst_start;   // first node of each instance (+ nnodes); {0, nnodes} for one mesh
     std::vector<int> inst_elem_start;   // first element of each instance (+ nelem) when contiguous, else empty
     ogb::DBuf<int> d_inst_start, d_inst_elem_start, d_node_inst;

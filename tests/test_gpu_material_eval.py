@@ -118,3 +118,41 @@ def test_plastic_evaluation_is_exercised():
     growth = [(gi[f"s{k}_omega"] > gi[f"s{k - 1}_omega"]) & (gi[f"s{k - 1}_omega"] > 0)
               for k in range(2, int(gi["nsteps"]) + 1)]
     assert any(x.any() for x in onset) and any(x.any() for x in growth)
+
+
+@pytest.mark.parametrize("dims", [(1, 1, 1), (3, 1, 1), (5, 1, 1), (4, 3, 3), (33, 1, 1), (7, 5, 2)])
+@pytest.mark.parametrize("material", ["isole", "mises", "idm1"])
+def test_hex_forces_and_tangent_sizes(dims, material, ctx, native_lib, oracle):
+    """LSpace internal forces, Gauss-point state and tangents by the elements' tensor
+    structure at sizes around a warp (four elements) and a block (32), every
+    material, against the oracle's full products: the same sums in another order,
+    so within 1e-12 of the field's maximum."""
+    from oofem_gb300 import meshgen as mg
+    mat = {"isole": mg.Material(mg.MAT_ISOLE, 210e9, 0.3), "mises": mg.Material(mg.MAT_MISES, 210e9, 0.3, sig0=250e6, H=2e9),
+           "idm1": mg.Material(mg.MAT_IDM1, 30e9, 0.2, e0=1e-4, gf=100.0)}[material]
+    mesh = mg.hex_block_pull(*dims, jitter=0.15, seed=2, material=mat)
+    scale = 2.0 * 250e6 / 210e9 if material != "idm1" else 2e-4
+    rng = np.random.default_rng(4)
+    u = mesh.coords * scale * np.array([1.0, -0.3, -0.3]) * (0.3 + mesh.coords[:, :1] / mesh.coords[:, 0].max())
+    u = u + rng.uniform(-0.02, 0.02, u.shape) * scale * 0.05
+    model = native_lib.GpuModel(ctx, mesh)
+    d = oracle.mesh_dict(mesh)
+    state = np.zeros((mesh.nelem * 8, 24))
+    # the damage law passes strains through a cubic's roots and an exponential
+    tol = 1e-10 if material == "idm1" else 1e-12
+    for k, s in enumerate((0.7, 1.0)):   # two increments: a committed state, then loading from it
+        f = model.internal_forces(s * u)
+        ref = oracle.internal_forces(d, s * u, None if material == "isole" else state)
+        assert rel(f, ref[0]) < tol, rel(f, ref[0])
+        sig, eps = model.gp_stress()
+        assert rel(sig.reshape(ref[1].shape), ref[1]) < tol and rel(eps.reshape(ref[2].shape), ref[2]) < tol
+        if material != "isole" and k == 0:
+            model.commit_state()
+            oracle.commit_state(d, state)
+    A = native_lib.GpuCsrMtrx(ctx)
+    model.build_matrix(A)
+    model.assemble_stiffness(A)
+    rp, ci = A.pattern()
+    neq, _, eq = oracle.number_equations(mesh.bc_mask)
+    K = oracle.assemble_tangent(d, oracle.location_arrays(mesh.conn, eq), neq, rp, ci, None if material == "isole" else state)
+    assert rel(A.values(), K) < tol, rel(A.values(), K)
