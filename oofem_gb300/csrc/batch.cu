@@ -71,19 +71,23 @@ __device__ __forceinline__ bool publish_inst(const double (&v)[NV], double *part
     return s_last;
 }
 
-// Fixed-order sums of the partials of units [u0, u1): thread t takes units
-// u0+t, u0+t+256, ..., then the fixed-order block reduction. Valid in thread 0.
+// Fixed-order sums of the partials of units [u0, u1), one value per warp (see
+// block_sum for why); returned in shared memory, for every thread.
 template <int NV>
-__device__ __forceinline__ void inst_sums(const double *part, int64_t u0, int64_t u1, double (&out)[NV])
+__device__ __forceinline__ const double *inst_sums(const double *part, int64_t u0, int64_t u1)
 {
+    __shared__ double tot[NV];
+    const int lane = threadIdx.x & 31;
     __threadfence();
-#pragma unroll
-    for (int k = 0; k < NV; ++k) out[k] = 0.0;
+    for (int k = threadIdx.x >> 5; k < NV; k += NTHREADS / 32) {
+        double s = 0.0;
 #pragma unroll 4
-    for (int64_t u = u0 + threadIdx.x; u < u1; u += NTHREADS)
-#pragma unroll
-        for (int k = 0; k < NV; ++k) out[k] += __ldcg(part + u * NV + k);
-    block_sum<NV>(out);
+        for (int64_t u = u0 + lane; u < u1; u += 32) s += __ldcg(part + u * NV + k);
+        s = warp_sum(s);
+        if (lane == 0) tot[k] = s;
+    }
+    __syncthreads();
+    return tot;
 }
 
 // Instance skip test (the same for every block of the instance within one
@@ -256,14 +260,12 @@ __global__ void __launch_bounds__(NTHREADS) k_bspmv(int nslices, const int64_t *
     double bs[NR];
     block_sum_t<NR, V>(dot, bs);
     if (!publish_inst<NR>(bs, part, blockIdx.x, cnt + inst, u1 - u0)) return;
-    double t[NR];
-    inst_sums<NR>(part, u0, u1, t);
-    if (threadIdx.x != 0) return;
-    cnt[inst] = 0;
-#pragma unroll
-    for (int c = 0; c < NR; ++c) {
+    const double *t = inst_sums<NR>(part, u0, u1);
+    if (threadIdx.x == 0) cnt[inst] = 0;
+    const int c = threadIdx.x;   // a thread per pair: their roots and divisions side by side
+    if (c < NR) {
         BatchScal &q = sc[inst * NR + c];
-        if (!pair_running<NR>(q)) continue;
+        if (!pair_running<NR>(q)) return;
         q.pq = t[c];
         if (!(t[c] > 0.0) || !isfinite(t[c])) q.done = sizeof(V) == 4 ? 5 : 2;   // FP32: the FP64 pass takes over
         else q.alpha = q.rho / t[c];
@@ -304,12 +306,10 @@ __global__ void __launch_bounds__(NTHREADS) k_binit(const double *__restrict__ b
     const int64_t u0 = unit_ptr[inst], u1 = unit_ptr[inst + 1];
     block_sum<3 * NR>(v);
     if (!publish_inst<3 * NR>(v, part, blockIdx.x, cnt + inst, u1 - u0)) return;
-    double t[3 * NR];
-    inst_sums<3 * NR>(part, u0, u1, t);
-    if (threadIdx.x != 0) return;
-    cnt[inst] = 0;
-#pragma unroll
-    for (int c = 0; c < NR; ++c) {
+    const double *t = inst_sums<3 * NR>(part, u0, u1);
+    if (threadIdx.x == 0) cnt[inst] = 0;
+    const int c = threadIdx.x;   // a thread per pair: their roots and divisions side by side
+    if (c < NR) {
         BatchScal &s = sc[inst * NR + c];
         s.bnorm2 = t[c];
         s.rnorm2 = t[NR + c];
@@ -365,14 +365,12 @@ __global__ void __launch_bounds__(NTHREADS) k_bupdate(double *__restrict__ x, do
     const int64_t u0 = unit_ptr[inst], u1 = unit_ptr[inst + 1];
     block_sum<2 * NR>(v);
     if (!publish_inst<2 * NR>(v, part, blockIdx.x, cnt + inst, u1 - u0)) return;
-    double t[2 * NR];
-    inst_sums<2 * NR>(part, u0, u1, t);
-    if (threadIdx.x != 0) return;
-    cnt[inst] = 0;
-#pragma unroll
-    for (int c = 0; c < NR; ++c) {
+    const double *t = inst_sums<2 * NR>(part, u0, u1);
+    if (threadIdx.x == 0) cnt[inst] = 0;
+    const int c = threadIdx.x;   // a thread per pair: their roots and divisions side by side
+    if (c < NR) {
         BatchScal &s = sc[inst * NR + c];
-        if (s.done) continue;
+        if (s.done) return;
         s.rnorm2 = t[c];
         s.iters += 1;
         double normb = sqrt(s.bnorm2);
@@ -537,14 +535,12 @@ __global__ void __launch_bounds__(NTHREADS) k_breplace(const double *__restrict_
     const int64_t u0 = unit_ptr[inst], u1 = unit_ptr[inst + 1];
     block_sum<3 * NR>(v);
     if (!publish_inst<3 * NR>(v, part, blockIdx.x, cnt + inst, u1 - u0)) return;
-    double t[3 * NR];
-    inst_sums<3 * NR>(part, u0, u1, t);
-    if (threadIdx.x != 0) return;
-    cnt[inst] = 0;
-#pragma unroll
-    for (int c = 0; c < NR; ++c) {
+    const double *t = inst_sums<3 * NR>(part, u0, u1);
+    if (threadIdx.x == 0) cnt[inst] = 0;
+    const int c = threadIdx.x;   // a thread per pair: their roots and divisions side by side
+    if (c < NR) {
         BatchScal &s = sc[inst * NR + c];
-        if (s.done || !(init || s.pause)) continue;
+        if (s.done || !(init || s.pause)) return;
         if (init) {
             s.bnorm2 = t[c];
             s.iters = 0;
@@ -627,14 +623,12 @@ __global__ void __launch_bounds__(NTHREADS) k_bupdate32(XS *__restrict__ x, floa
     double bs[2 * NR];
     block_sum_t<2 * NR, float>(v, bs);
     if (!publish_inst<2 * NR>(bs, part, blockIdx.x, cnt + inst, u1 - u0)) return;
-    double t[2 * NR];
-    inst_sums<2 * NR>(part, u0, u1, t);
-    if (threadIdx.x != 0) return;
-    cnt[inst] = 0;
-#pragma unroll
-    for (int c = 0; c < NR; ++c) {
+    const double *t = inst_sums<2 * NR>(part, u0, u1);
+    if (threadIdx.x == 0) cnt[inst] = 0;
+    const int c = threadIdx.x;   // a thread per pair: their roots and divisions side by side
+    if (c < NR) {
         BatchScal &s = sc[inst * NR + c];
-        if (!pair_running<NR>(s)) continue;
+        if (!pair_running<NR>(s)) return;
         s.rnorm2 = t[c];
         s.iters += 1;
         s.repl = 0;

@@ -20,36 +20,47 @@ __device__ __forceinline__ T warp_sum(T v)
 }
 
 // Fixed-order block reduction of NV values per thread; result valid in thread 0.
+// The threads' values go through shared memory and warp k adds value k: eight
+// additions per lane and five shuffles. FP64 additions are what a reduction costs
+// on this part (a warp's instruction holds a quarter of the SM's FP64 pipe for 64
+// cycles): shuffles in all eight warps and a serial sum over the warps took 48 per
+// value, this takes 12, and several values run side by side.
 template <int NV>
 __device__ __forceinline__ void block_sum(double (&v)[NV])
 {
-    __shared__ double red[NV][NTHREADS / 32];
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int W = NTHREADS / 32;
+    __shared__ double st[NV][NTHREADS], res[NV];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        double s = warp_sum(v[k]);
-        if (lane == 0) red[k][warp] = s;
+    for (int k = 0; k < NV; ++k) st[k][threadIdx.x] = v[k];
+    __syncthreads();
+    for (int k = warp; k < NV; k += W) {
+        const double *q = st[k] + lane;
+        static_assert(W == 8, "the tree below adds eight values");
+        double s = ((q[0] + q[32]) + (q[64] + q[96])) + ((q[128] + q[160]) + (q[192] + q[224]));
+        s = warp_sum(s);
+        if (lane == 0) res[k] = s;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0)
 #pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            double s = 0;
-#pragma unroll
-            for (int w = 0; w < NTHREADS / 32; ++w) s += red[k][w];
-            v[k] = s;
-        }
-    }
-    __syncthreads();
+        for (int k = 0; k < NV; ++k) v[k] = res[k];
 }
 
 // Block reduction of per-thread values of type T: the warp sum stays in T (an
 // FP32 warp sum costs no FP64 instruction), the warps are added in FP64 in
-// index order. Result valid in thread 0.
+// index order, one value per lane (in one thread value after value the additions
+// alone took 24 us of the batched SpMV's first SM partition). Result valid in thread 0.
 template <int NV, class T>
 __device__ __forceinline__ void block_sum_t(const T (&v)[NV], double (&out)[NV])
 {
-    __shared__ double red[NV][NTHREADS / 32];
+    if constexpr (sizeof(T) == 8) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) out[k] = v[k];
+        block_sum<NV>(out);
+        return;
+    }
+    __shared__ double red[NV][NTHREADS / 32], res[NV];
     int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
@@ -57,14 +68,17 @@ __device__ __forceinline__ void block_sum_t(const T (&v)[NV], double (&out)[NV])
         if (lane == 0) red[k][warp] = (double)s;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
+    if (warp == 0) {
+        if (lane < NV) {
             double s = 0;
 #pragma unroll
-            for (int w = 0; w < NTHREADS / 32; ++w) s += red[k][w];
-            out[k] = s;
+            for (int w = 0; w < NTHREADS / 32; ++w) s += red[lane][w];
+            res[lane] = s;
         }
+        __syncwarp();
+        if (lane == 0)
+#pragma unroll
+            for (int k = 0; k < NV; ++k) out[k] = res[k];
     }
     __syncthreads();
 }
