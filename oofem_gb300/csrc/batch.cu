@@ -35,18 +35,6 @@ namespace ogb {
 
 namespace {
 
-struct BatchScal {
-    double bnorm2, rho, pq, rnorm2, alpha, beta;
-    double mark;   // mixed precision: FP64 residual^2 at the last halving
-    double rrep;   // mixed precision: FP64 residual^2 at the last replacement (the drop test's reference)
-    int done;      // 0 running, 1 converged, 2 breakdown, 3 zero pivot, 4 iteration limit, 5 stalled (mixed)
-    int iters;
-    int pause;     // mixed precision: waits for the next FP64 residual replacement
-    int since;     // mixed precision: replacements since the FP64 residual last halved
-    int repl;      // mixed precision: replaced in the last replacement pass, p update pending
-    int pad_;
-};
-
 constexpr int RPT = 4;                       // scalar rows per thread in the vector kernels
 constexpr int UNIT = RPT * NTHREADS;         // scalar rows per vector block (1024)
 constexpr int SPMV_SLICES = NTHREADS / 32;   // slices (of 32 node rows) per SpMV block
@@ -811,6 +799,9 @@ int run_batch(ogb_mtrx *m, const double *b, double *x, double rtol, int maxit, b
             w.sptr.p, skip);
     };
     std::function<void()> iteration;
+    // small batches: every instance's iterations (and its residual replacements) in one launch
+    BatchPersistPlan plan;
+    const bool persist = batch_persist_plan(ctx, S, NR, mixed, plan);
     // mixed preconditioner: FP32 block Jacobi of the 2 x 2 node blocks (two DOFs
     // per node) where the option allows it, else the scalar diagonal
     const bool bj2 = mixed && ND == 2 && ctx->mixed_bj;
@@ -853,7 +844,7 @@ int run_batch(ogb_mtrx *m, const double *b, double *x, double rtol, int maxit, b
         };
         SellMat &Sm = const_cast<SellMat &>(S);
         if (ctx->batch_form) Sm.bform32 = ctx->batch_form;
-        if (!Sm.bform32) {
+        if (!Sm.bform32 && !persist) {
             cudaEvent_t e0, e1;
             OGB_CUDA(cudaEventCreate(&e0));
             OGB_CUDA(cudaEventCreate(&e1));
@@ -880,7 +871,7 @@ int run_batch(ogb_mtrx *m, const double *b, double *x, double rtol, int maxit, b
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
         }
-        const int bform = Sm.bform32;
+        const int bform = Sm.bform32 ? Sm.bform32 : 1;
         // with kernel timing on, one more launch of the chosen form on the first
         // search directions is timed when every pair is running (no instance
         // skipped): the launch recomputes q, p.q and alpha of the same p, so the
@@ -948,7 +939,7 @@ int run_batch(ogb_mtrx *m, const double *b, double *x, double rtol, int maxit, b
     count_launch(ctx, 3);
     OGB_CUDA(cudaGetLastError());
     ExecGuard graph;
-    OGB_CHECK(capture_batch(ctx, iteration, graph.e));
+    if (!persist) OGB_CHECK(capture_batch(ctx, iteration, graph.e));
     int zero = 0;
     OGB_CUDA(cudaMemcpyAsync(&zero, w.zero.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     res.resize(npair);
@@ -959,12 +950,24 @@ int run_batch(ogb_mtrx *m, const double *b, double *x, double rtol, int maxit, b
             for (auto &s : res) s.done = 3;
             break;
         }
+        for (auto &s : res)
+            if (s.done == BATCH_WAIT_TIMEOUT)
+                return fail(OGB_E_CUDA, "batched CG iterations: the blocks did not all arrive within the wait limit");
         bool all = true, paused = false;
         for (auto &s : res) {
             all = all && s.done;
             paused = paused || (s.done == 0 && s.pause != 0);
         }
-        if (all || it > maxit + 2 * BBATCH) break;
+        if (all || it > maxit + 2 * (persist ? plan.budget : BBATCH)) break;
+        if (persist) {
+            OGB_CHECK(batch_persist_run(m, plan, NR, mixed, b, x, mixed ? (void *)w.r32.p : (void *)w.r.p,
+                                        mixed ? (void *)w.z32.p : (void *)w.z.p, mixed ? (void *)w.p32.p : (void *)w.p.p,
+                                        mixed ? (void *)w.q32.p : (void *)w.q.p,
+                                        bj2 ? (const void *)w.binv2.p : mixed ? (const void *)w.dinv32.p : (const void *)w.dinv.p,
+                                        bj2, w.sc.p, rtol, maxit, ctx->mixed_drop * ctx->mixed_drop));
+            it += plan.budget;
+            continue;
+        }
         if (mixed && paused) {
             // FP64 replacement of the pairs that paused during the last batch of
             // iterations (instances without one skip every kernel): residual, r, z,

@@ -121,6 +121,20 @@ struct PcgScal {
     int cycle_end;    // mixed: iteration count at which the current cycle ends at the latest
 };
 
+// Scalars of one (instance, right-hand side) pair of a batched solve (batch.cu).
+struct BatchScal {
+    double bnorm2, rho, pq, rnorm2, alpha, beta;
+    double mark;   // mixed precision: FP64 residual^2 at the last halving
+    double rrep;   // mixed precision: FP64 residual^2 at the last replacement (the drop test's reference)
+    int done;      // 0 running, 1 converged, 2 breakdown, 3 zero pivot, 4 iteration limit, 5 stalled (mixed),
+                   // 6 a wait of the one-launch form timed out
+    int iters;
+    int pause;     // mixed precision: waits for the next FP64 residual replacement
+    int since;     // mixed precision: replacements since the FP64 residual last halved
+    int repl;      // mixed precision: replaced in the last replacement pass, p update pending
+    int pad_;
+};
+
 // Node-block SELL-32 storage: rows = active nodes (>= 1 free DOF) in node
 // order, ND x ND blocks, 32 rows per slice, blocks of a slice stored k-major so
 // that lane r of a warp reads row r's k-th block with coalesced loads.
@@ -173,6 +187,7 @@ struct SellMat {
     int group[2] = {0, 0};  // tuned SpMV variant for FP64 / FP32 values (0 = not yet)
     int force_split = 0;    // warps per slice forced by OGB_OPT_SPMV_VARIANT 5 / 6 (0 = rule)
     int bform32 = 0;        // batched FP32 SpMV form timed for this matrix: 1 plain, 2 values of a group first
+    std::vector<int> inst_nact;           // active node rows of each instance
     std::vector<int64_t> inst_row_base;   // first node-space row of each instance (+ total)
     HalfSell half;                        // half-stored FP32 copy (built on first use)
     int64_t nns() const { return (int64_t)nslices * 32 * nd; }
@@ -297,6 +312,8 @@ struct ogb_mtrx {
     ogb::HBuf<ogb::PcgScal> h_scal;
     ogb::DBuf<unsigned int> w_count;
     ogb::DBuf<double> w_mail;                    // mailboxes of the one-launch iterations (persist.cu)
+    ogb::DBuf<double> w_bmail;                   // ... of batches (persist_batch.cu)
+    ogb::DBuf<int> w_bcta;                       // ... and what each of their CTAs works on
     unsigned long long mail_epoch = 0;           // last exchange posted to them
     ogb::DBuf<unsigned int> w_epoch;             // fused update: advanced once per iteration by its last block
     int spmv_tpr = 8;    // threads per row of the CSR SpMV (autotuned)
@@ -431,6 +448,17 @@ struct PersistPlan {
 bool persist_plan(const ogb_ctx *ctx, const SellMat &S, bool mixed, PersistPlan &P);
 int persist_run(ogb_mtrx *m, const PersistPlan &P, bool mixed, const void *val, double *x, void *r, void *p, void *z,
                 void *p2, const void *prec, double rtol, int maxit);
+
+// persist_batch.cu: the same for the instances of a small batch.
+constexpr int BATCH_WAIT_TIMEOUT = 6;   // BatchScal::done
+struct BatchPersistPlan {
+    int rows = 0, grid = 0, nt = 0, rpt = 1, kmax = 0, kc = 0, budget = 512;
+    size_t smem = 0;
+    std::vector<int> cta;   // per CTA: instance, first CTA and CTAs of the instance, first row, end of the instance's rows
+};
+bool batch_persist_plan(const ogb_ctx *ctx, const SellMat &S, int nr, bool mixed, BatchPersistPlan &P);
+int batch_persist_run(ogb_mtrx *m, const BatchPersistPlan &P, int nr, bool mixed, const double *b, double *x, void *r, void *z,
+                      void *p, void *p2, const void *prec, bool blocks2, BatchScal *sc, double rtol, int maxit, double drop2);
 
 // direct.cu: LDL^T factor of m (cached per version) and x = A^-1 b on padded
 // equation-space device vectors (info: 0 iterations, FP64 relative residual).

@@ -695,9 +695,11 @@ int build_sell(ogb_model *md, ogb_mtrx *m)
     OGB_CUDA(cudaStreamSynchronize(st));
     std::vector<int64_t> rank0(ninst), base(ninst + 1, 0);
     S.inst_row_base.assign(ninst + 1, 0);
+    S.inst_nact.assign(ninst, 0);
     for (int i = 0; i < ninst; ++i) {
         rank0[i] = rank[md->inst_start[i]];
         int64_t na = rank[md->inst_start[i + 1]] - rank0[i];
+        S.inst_nact[i] = (int)na;
         base[i + 1] = base[i] + ceil_div(na > 0 ? na : 1, INST_ALIGN) * INST_ALIGN;
     }
     S.inst_row_base = base;

@@ -1,0 +1,536 @@
+// Iterations of a small batch in one launch (see persist.cu for the scheme).
+//
+// Every instance gets CTAs of its own, as many as its node rows need, and advances
+// all its load cases by itself: a group of CTAs exchanges its sums through its own
+// mailboxes and does not wait for other instances; an instance of one CTA needs no
+// exchange at all. In mixed solves a pair whose recursive residual has dropped (the
+// batched update's test) has it replaced by b - K64 x right away in the same launch,
+// by its own group, where the multi-launch form goes through the host and three
+// kernels over the whole batch for every round of replacements (18 of them per solve
+// of the IDM1 cubes); the pair goes on from the same p = z + beta p. x is kept in
+// FP64 throughout.
+//
+// Measured (GB300): four IDM1 cubes of 10^3 cells (16 k rows), 20.4 k iterations and 1,023
+// rounds of replacements: 18.2 us an iteration and 70 us a round -> 6.9 us in all.
+#include <math.h>
+
+#include <algorithm>
+
+#include "persist.cuh"
+
+namespace ogb {
+
+namespace {
+
+struct BatchArgs {
+    int kmax, kc, cw;                     // blocks per thread, of them in shared memory; ints per CTA record
+    const int *cta;
+    const int64_t *sl_ptr;
+    const int *sl_width, *col;
+    const void *val;
+    const double *val64, *b;
+    double *x;
+    void *r, *z, *p, *p2;
+    const void *prec;                     // inverse diagonal by scalar row, or rows of the 2 x 2 inverses
+    Mail *mail;
+    unsigned long long epoch;
+    BatchScal *sc;
+    double rtol, drop2;
+    int maxit, budget;
+};
+
+// T: double (IML CG per pair) or float (mixed). RPT: node rows per group of four
+// threads; a thread holds degree of freedom `part` of its rows, for all load cases.
+template <int ND, int NR, class T, int RPT, bool BJ2>
+__global__ void __launch_bounds__(512, 1) k_batch_persist(BatchArgs a)
+{
+    constexpr bool MIXED = sizeof(T) == 4;
+    constexpr int NB = ND * ND, W = ND * NR, MV = 2 * NR;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ double warp_sums[4 * 3 * NR];
+    __shared__ BatchScal S[NR];
+    __shared__ bool fine;
+    const int nt = blockDim.x, t = threadIdx.x, part = t & 3, lane = t & 31, group = t >> 2, groups = nt >> 2;
+    const int *rec = a.cta + (size_t)blockIdx.x * a.cw;
+    const int inst = rec[0], first_cta = rec[1], G = rec[2], row0 = rec[3], row1 = rec[4];
+    const T *val = static_cast<const T *>(a.val);
+    T *r_g = static_cast<T *>(a.r), *z_g = static_cast<T *>(a.z);
+    T *p_old = static_cast<T *>(a.p2), *p_new = static_cast<T *>(a.p);
+    if (t < NR) S[t] = a.sc[inst * NR + t];
+    if (t == 0) fine = true;
+    __syncthreads();
+    bool any = false;
+#pragma unroll
+    for (int c = 0; c < NR; ++c) any |= S[c].done == 0;
+    if (!any) return;   // the same in every CTA of the instance
+    // shared memory: this thread's matrix blocks, then the terms of the sums
+    T *sv = reinterpret_cast<T *>(smem);
+    int *scol = reinterpret_cast<int *>(smem + (size_t)RPT * a.kc * NB * nt * sizeof(T));
+    double *terms = reinterpret_cast<double *>(smem + (((size_t)RPT * a.kc * nt * (NB * sizeof(T) + 4) + 15) & ~(size_t)15));
+    int row[RPT];
+    bool mine[RPT];
+    int64_t slot0[RPT];
+    int width[RPT];
+    double x[RPT][NR];
+    T r[RPT][NR], z[RPT][NR], p[RPT][NR], d0[RPT], d1[RPT];
+#pragma unroll
+    for (int rp = 0; rp < RPT; ++rp) {
+        const int q = row0 + group + rp * groups;
+        const bool on = q < row1;
+        row[rp] = on ? q : row0;
+        slot0[rp] = a.sl_ptr[row[rp] >> 5] + (row[rp] & 31);
+        width[rp] = on ? a.sl_width[row[rp] >> 5] : 0;
+        mine[rp] = on && part < ND;
+        const int64_t sr = (int64_t)row[rp] * ND + (part < ND ? part : 0);
+        d0[rp] = d1[rp] = 0;
+        if (mine[rp]) {
+            if constexpr (BJ2) {
+                const float2 v = static_cast<const float2 *>(a.prec)[sr];
+                d0[rp] = v.x;
+                d1[rp] = v.y;
+            } else {
+                d0[rp] = static_cast<const T *>(a.prec)[sr];
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < NR; ++c) {
+            const int64_t i = sr * NR + c;
+            x[rp][c] = mine[rp] ? a.x[i] : 0.0;
+            r[rp][c] = mine[rp] ? r_g[i] : (T)0;
+            p[rp][c] = mine[rp] ? p_new[i] : (T)0;
+            z[rp][c] = 0;
+        }
+        for (int k = 0; k < a.kc; ++k) {
+            const int kk = k * PARTS + part;
+            const bool has = kk < width[rp];
+            const int64_t slot = slot0[rp] + 32 * (int64_t)kk;
+            scol[(size_t)(rp * a.kc + k) * nt + t] = has ? a.col[slot] : row[rp];
+            const T *v = val + (slot - (row[rp] & 31)) * NB + (row[rp] & 31);
+#pragma unroll
+            for (int e = 0; e < NB; ++e) sv[((size_t)(rp * a.kc + k) * NB + e) * nt + t] = has ? __ldcs(v + 32 * e) : (T)0;
+        }
+    }
+    // component `part` of the sums over the four threads of a row (see persist.cu)
+    auto fold = [&](auto (&y)[ND]) {
+        using Y = std::remove_reference_t<decltype(y[0])>;
+        if constexpr (ND == 3) {
+            const Y y2 = __shfl_xor_sync(0xffffffffu, part < 2 ? y[2] : y[0], 2);
+            const Y y1 = __shfl_xor_sync(0xffffffffu, y[1], 2);
+            const Y h0 = (part < 2 ? y[0] : y[2]) + y2, h1 = y[1] + y1;
+            const Y give = __shfl_xor_sync(0xffffffffu, part == 0 ? h1 : h0, 1);
+            return (part == 1 ? h1 : h0) + give;
+        } else {
+            const Y give = __shfl_xor_sync(0xffffffffu, part & 1 ? y[0] : y[1], 1);
+            const Y h = (part & 1 ? y[1] : y[0]) + give;
+            return h + __shfl_xor_sync(0xffffffffu, h, 2);
+        }
+    };
+    auto precondition = [&](T res, int rp) -> T {   // called by all lanes
+        if constexpr (BJ2) {
+            const T other = __shfl_xor_sync(0xffffffffu, res, 1);
+            return fmaf(d1[rp], part & 1 ? res : other, d0[rp] * (part & 1 ? other : res));
+        } else {
+            return res * d0[rp];
+        }
+    };
+    unsigned long long epoch = a.epoch;
+    bool first = true;
+    bool run[NR];
+    T beta[NR];
+#pragma unroll
+    for (int c = 0; c < NR; ++c) {
+        run[c] = S[c].done == 0;
+        beta[c] = 0;
+    }
+    for (int it = 0;; ++it) {
+        // q = K p of the running pairs
+        T q[RPT][NR], pq[NR];
+#pragma unroll
+        for (int c = 0; c < NR; ++c) pq[c] = 0;
+#pragma unroll
+        for (int rp = 0; rp < RPT; ++rp) {
+            T y[NR][ND], pa[NR][ND];
+#pragma unroll
+            for (int c = 0; c < NR; ++c)
+#pragma unroll
+                for (int i = 0; i < ND; ++i) {
+                    y[c][i] = 0;
+                    pa[c][i] = MIXED ? __shfl_sync(0xffffffffu, p[rp][c], (lane & ~3) + i) : (T)0;
+                }
+            auto product = [&](int col, const T (&v)[NB]) {
+                T pc[W];
+                const int64_t i0 = (int64_t)col * W;
+#pragma unroll
+                for (int j = 0; j < W; ++j) {
+                    pc[j] = first ? p_new[i0 + j] : fma(beta[j % NR], p_old[i0 + j], z_g[i0 + j]);
+                    if (MIXED && col != row[rp]) pc[j] -= pa[j % NR][j / NR];
+                }
+#pragma unroll
+                for (int c = 0; c < NR; ++c)
+#pragma unroll
+                    for (int i = 0; i < ND; ++i)
+#pragma unroll
+                        for (int j = 0; j < ND; ++j) y[c][i] = fma(v[i * ND + j], pc[j * NR + c], y[c][i]);
+            };
+#pragma unroll 2
+            for (int k = 0; k < a.kc; ++k) {
+                T v[NB];
+#pragma unroll
+                for (int e = 0; e < NB; ++e) v[e] = sv[((size_t)(rp * a.kc + k) * NB + e) * nt + t];
+                product(scol[(size_t)(rp * a.kc + k) * nt + t], v);
+            }
+            for (int k = a.kc; k < a.kmax; ++k) {
+                const int kk = k * PARTS + part;
+                if (kk >= width[rp]) break;
+                const int64_t slot = slot0[rp] + 32 * (int64_t)kk;
+                const T *vp = val + (slot - (row[rp] & 31)) * NB + (row[rp] & 31);
+                T v[NB];
+#pragma unroll
+                for (int e = 0; e < NB; ++e) v[e] = __ldg(vp + 32 * e);
+                product(__ldg(a.col + slot), v);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < NR; ++c) {
+                q[rp][c] = fold(y[c]);
+                if (mine[rp]) pq[c] = fma(p[rp][c], q[rp][c], pq[c]);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < NR; ++c) terms[c * nt + t] = (double)pq[c];
+        double s0[NR], s1[NR];
+        cta_sum<NR>(terms, nt, nt, s0, warp_sums);
+        if (t < 32) {
+            const bool ok = exchange<NR, false, MV>(a.mail, epoch, first_cta, G, s0, s1);
+            if (t == 0) fine = ok;
+#pragma unroll
+            for (int c = 0; c < NR; ++c)
+                if (t == c && run[c]) {
+                    S[c].pq = s1[c];
+                    if (!(s1[c] > 0.0) || !isfinite(s1[c])) S[c].done = MIXED ? 5 : 2;   // FP32: the FP64 pass takes over
+                    else S[c].alpha = S[c].rho / s1[c];
+                }
+        }
+        ++epoch;
+        __syncthreads();
+        if (!fine) break;
+#pragma unroll
+        for (int c = 0; c < NR; ++c) run[c] = run[c] && S[c].done == 0;
+        // x, r, z of the running pairs; r.r and r.z
+        T rr[NR], rz[NR];
+#pragma unroll
+        for (int c = 0; c < NR; ++c) {
+            rr[c] = rz[c] = 0;
+            if (!run[c]) continue;
+            const double alpha = S[c].alpha;
+#pragma unroll
+            for (int rp = 0; rp < RPT; ++rp) {
+                x[rp][c] = fma(alpha, (double)p[rp][c], x[rp][c]);
+                r[rp][c] = mine[rp] ? fma(-(T)alpha, q[rp][c], r[rp][c]) : (T)0;
+                z[rp][c] = precondition(r[rp][c], rp);
+                rr[c] = fma(r[rp][c], r[rp][c], rr[c]);
+                if (mine[rp]) {
+                    rz[c] = fma(r[rp][c], z[rp][c], rz[c]);
+                    z_g[((int64_t)row[rp] * ND + part) * NR + c] = z[rp][c];
+                }
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < NR; ++c) {
+            terms[c * nt + t] = (double)rr[c];
+            terms[(NR + c) * nt + t] = (double)rz[c];
+        }
+        double t0[2 * NR], t1[2 * NR];
+        cta_sum<2 * NR>(terms, nt, nt, t0, warp_sums);
+        if (t < 32) {
+            const bool ok = exchange<2 * NR, true, MV>(a.mail, epoch, first_cta, G, t0, t1);
+            if (t == 0) fine = ok;
+#pragma unroll
+            for (int c = 0; c < NR; ++c)
+                if (t == c && run[c]) {
+                    BatchScal &s = S[c];
+                    s.rnorm2 = t1[c];
+                    s.iters += 1;
+                    s.repl = 0;
+                    double normb = sqrt(s.bnorm2);
+                    if (normb == 0.0) normb = 1.0;
+                    if (MIXED) {
+                        const double half = 0.5 * a.rtol * normb;
+                        if (!isfinite(t1[c]) || !isfinite(t1[NR + c])) s.done = 5;
+                        else if (t1[c] <= half * half || t1[c] <= a.drop2 * s.rrep || !(t1[NR + c] > 0.0) || s.iters >= a.maxit)
+                            s.pause = 1;
+                    } else {
+                        if (sqrt(t1[c]) / normb <= a.rtol) s.done = 1;
+                        else if (!isfinite(t1[NR + c]) || !(t1[NR + c] > 0.0)) s.done = 2;
+                        else if (s.iters >= a.maxit) s.done = 4;
+                    }
+                    if (!s.done && !s.pause) {
+                        s.beta = t1[NR + c] / s.rho;
+                        s.rho = t1[NR + c];
+                    }
+                }
+        }
+        ++epoch;
+        __syncthreads();
+        if (!fine) break;
+        if constexpr (MIXED) {
+            bool paused[NR], some = false;
+#pragma unroll
+            for (int c = 0; c < NR; ++c) {
+                paused[c] = run[c] && S[c].pause != 0;
+                some |= paused[c];
+            }
+            if (some) {
+                // r = b - K64 x of the paused pairs, by the same threads from the FP64 copy
+#pragma unroll
+                for (int rp = 0; rp < RPT; ++rp)
+                    if (mine[rp])
+#pragma unroll
+                        for (int c = 0; c < NR; ++c)
+                            if (paused[c]) a.x[((int64_t)row[rp] * ND + part) * NR + c] = x[rp][c];
+                __syncthreads();
+                if (t < 32) {
+                    const double none[1] = {0.0};
+                    double got[1];
+                    const bool ok = exchange<1, true, MV>(a.mail, epoch, first_cta, G, none, got);
+                    if (t == 0) fine = ok;
+                }
+                ++epoch;
+                __syncthreads();
+                if (!fine) break;
+                double n6[NR], nz[NR];
+#pragma unroll
+                for (int c = 0; c < NR; ++c) {
+                    n6[c] = nz[c] = 0.0;
+                    if (!paused[c]) continue;
+#pragma unroll
+                    for (int rp = 0; rp < RPT; ++rp) {
+                        double y[ND];
+#pragma unroll
+                        for (int i = 0; i < ND; ++i) y[i] = 0.0;
+                        for (int k = 0; k < a.kmax; ++k) {
+                            const int kk = k * PARTS + part;
+                            if (kk >= width[rp]) break;
+                            const int64_t slot = slot0[rp] + 32 * (int64_t)kk;
+                            const double *vp = a.val64 + (slot - (row[rp] & 31)) * NB + (row[rp] & 31);
+                            const int64_t i0 = (int64_t)__ldg(a.col + slot) * W + c;
+                            double xc[ND];
+#pragma unroll
+                            for (int j = 0; j < ND; ++j) xc[j] = a.x[i0 + j * NR];
+#pragma unroll
+                            for (int i = 0; i < ND; ++i)
+#pragma unroll
+                                for (int j = 0; j < ND; ++j) y[i] = fma(__ldg(vp + 32 * (i * ND + j)), xc[j], y[i]);
+                        }
+                        __syncwarp();
+                        const double kx = fold(y);
+                        const double r6 = mine[rp] ? a.b[((int64_t)row[rp] * ND + part) * NR + c] - kx : 0.0;
+                        const T rf = (T)r6;
+                        r[rp][c] = rf;
+                        z[rp][c] = precondition(rf, rp);
+                        if (mine[rp]) {
+                            z_g[((int64_t)row[rp] * ND + part) * NR + c] = z[rp][c];
+                            n6[c] = fma(r6, r6, n6[c]);
+                            nz[c] += (double)(rf * z[rp][c]);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < NR; ++c) {
+                    terms[c * nt + t] = n6[c];
+                    terms[(NR + c) * nt + t] = nz[c];
+                }
+                cta_sum<2 * NR>(terms, nt, nt, t0, warp_sums);
+                if (t < 32) {
+                    const bool ok = exchange<2 * NR, true, MV>(a.mail, epoch, first_cta, G, t0, t1);
+                    if (t == 0) fine = ok;
+#pragma unroll
+                    for (int c = 0; c < NR; ++c)
+                        if (t == c && paused[c]) {   // the decisions of k_breplace
+                            BatchScal &s = S[c];
+                            double normb = sqrt(s.bnorm2);
+                            if (normb == 0.0) normb = 1.0;
+                            s.rnorm2 = t1[c];
+                            const double zr = t1[NR + c];
+                            if (t1[c] < 0.25 * s.mark) {
+                                s.mark = t1[c];
+                                s.since = 0;
+                            } else {
+                                ++s.since;
+                            }
+                            if (sqrt(t1[c]) / normb <= a.rtol) s.done = 1;
+                            else if (!isfinite(t1[c])) s.done = 2;
+                            else if (s.iters >= a.maxit) s.done = 4;
+                            else if (!isfinite(zr) || !(zr > 0.0) || s.since >= 6) s.done = 5;
+                            else {
+                                s.beta = zr / s.rho;
+                                s.rho = zr;
+                                s.rrep = t1[c];
+                                s.pause = 0;
+                            }
+                        }
+                }
+                ++epoch;
+                __syncthreads();
+                if (!fine) break;
+            }
+        }
+        any = false;
+#pragma unroll
+        for (int c = 0; c < NR; ++c) {
+            run[c] = run[c] && S[c].done == 0;
+            any |= run[c];
+            beta[c] = (T)S[c].beta;
+        }
+        if (!any) break;
+        first = false;
+        T *swap = p_old;
+        p_old = p_new;
+        p_new = swap;
+#pragma unroll
+        for (int rp = 0; rp < RPT; ++rp)
+#pragma unroll
+            for (int c = 0; c < NR; ++c) {
+                // (a pair that is done keeps no p: its products are not used)
+                p[rp][c] = fma(beta[c], p[rp][c], z[rp][c]);
+                if (mine[rp]) p_new[((int64_t)row[rp] * ND + part) * NR + c] = p[rp][c];
+            }
+        if (it + 1 == a.budget) break;
+    }
+#pragma unroll
+    for (int rp = 0; rp < RPT; ++rp)
+        if (mine[rp])
+#pragma unroll
+            for (int c = 0; c < NR; ++c) {
+                const int64_t i = ((int64_t)row[rp] * ND + part) * NR + c;
+                a.x[i] = x[rp][c];
+                r_g[i] = r[rp][c];
+                static_cast<T *>(a.p)[i] = p[rp][c];
+            }
+    if (fine) {
+        if (blockIdx.x == first_cta && t < NR) a.sc[inst * NR + t] = S[t];
+    } else if (t == 0) {
+        for (int c = 0; c < NR; ++c) a.sc[inst * NR + c].done = BATCH_WAIT_TIMEOUT;
+    }
+}
+
+template <int ND, int NR, class T, bool BJ2>
+const void *fn_rpt(int rpt)
+{
+    if (rpt == 1) return (const void *)k_batch_persist<ND, NR, T, 1, BJ2>;
+    if constexpr (sizeof(T) * NR <= 12) {
+        if (rpt == 2) return (const void *)k_batch_persist<ND, NR, T, 2, BJ2>;
+    }
+    if constexpr (sizeof(T) * NR <= 4) {
+        if (rpt <= 4) return (const void *)k_batch_persist<ND, NR, T, 4, BJ2>;
+    }
+    return nullptr;
+}
+
+template <int ND, class T, bool BJ2>
+const void *fn_nr(int nr, int rpt)
+{
+    switch (nr) {
+    case 1: return fn_rpt<ND, 1, T, BJ2>(rpt);
+    case 2: return fn_rpt<ND, 2, T, BJ2>(rpt);
+    case 3: return fn_rpt<ND, 3, T, BJ2>(rpt);
+    default: return fn_rpt<ND, 4, T, BJ2>(rpt);
+    }
+}
+
+constexpr int CTA_INTS = 5;
+constexpr int SMEM_MAX = 227 * 1024 - 2 * 1024;   // the kernel's own arrays: under 2 KB
+
+}  // namespace
+
+// Shape of the launch: the fewest rows per CTA with which every instance's CTAs fit
+// the device together. Several rows per thread only where the load cases' vectors
+// stay in registers (rpt x cases x bytes); beyond that the batch is large enough for
+// the streaming kernels.
+bool batch_persist_plan(const ogb_ctx *ctx, const SellMat &S, int nr, bool mixed, BatchPersistPlan &P)
+{
+    if (!ctx->persist || (mixed && !ctx->mixed_diff) || (mixed && !ctx->mixed_bj)) return false;
+    const int sms = std::min(num_sms(), MAX_CTAS);
+    if (S.ninst > sms || (int)S.inst_nact.size() != S.ninst) return false;
+    const int tb = mixed ? 4 : 8;
+    const int rptmax = tb * nr <= 4 ? 4 : tb * nr <= 12 ? 2 : 1;
+    const int limit = 128 * rptmax;
+    int rows = 8;
+    for (;; rows += 8) {
+        if (rows > limit) return false;
+        int64_t n = 0;
+        for (int v : S.inst_nact) n += std::max<int64_t>(1, ceil_div(v, rows));
+        if (n <= sms) break;
+    }
+    P.rows = rows;
+    P.rpt = (int)ceil_div(rows, 128);
+    if (P.rpt == 3) P.rpt = 4;
+    P.nt = (int)ceil_div(ceil_div(rows, P.rpt) * PARTS, 32) * 32;
+    P.kmax = (int)ceil_div(S.max_width, PARTS);
+    const int64_t block = (int64_t)S.nd * S.nd * tb + 4, sums = (int64_t)2 * nr * P.nt * 8 + 16;
+    P.kc = (int)std::min<int64_t>(P.kmax, (SMEM_MAX - sums) / (block * P.nt * P.rpt));
+    P.smem = (size_t)(block * P.nt * P.rpt * P.kc + sums);
+    P.cta.clear();
+    for (int i = 0; i < S.ninst; ++i) {
+        const int n = (int)std::max<int64_t>(1, ceil_div(S.inst_nact[i], rows)), first = (int)P.cta.size() / CTA_INTS;
+        const int base = (int)S.inst_row_base[i], end = base + S.inst_nact[i];
+        for (int k = 0; k < n; ++k) {
+            const int r0 = base + k * rows;
+            P.cta.insert(P.cta.end(), {i, first, n, r0, std::max(r0, std::min(r0 + rows, end))});
+        }
+    }
+    P.grid = (int)P.cta.size() / CTA_INTS;
+    return true;
+}
+
+int batch_persist_run(ogb_mtrx *m, const BatchPersistPlan &P, int nr, bool mixed, const double *b, double *x, void *r, void *z,
+                      void *p, void *p2, const void *prec, bool blocks2, BatchScal *sc, double rtol, int maxit, double drop2)
+{
+    ogb_ctx *ctx = m->ctx;
+    cudaStream_t s = ctx->stream;
+    const SellMat &S = m->sell;
+    const size_t boxes = (size_t)2 * 2 * nr * P.grid * P.grid;
+    if (m->w_bmail.n < 2 * boxes) {
+        OGB_CHECK(m->w_bmail.alloc(2 * boxes));
+        OGB_CUDA(cudaMemsetAsync(m->w_bmail.p, 0, m->w_bmail.n * sizeof(double), s));   // epoch 0: no exchange's
+    }
+    OGB_CHECK(m->w_bcta.alloc(P.cta.size()));
+    OGB_CUDA(cudaMemcpyAsync(m->w_bcta.p, P.cta.data(), P.cta.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+    BatchArgs a{};
+    a.kmax = P.kmax;
+    a.kc = P.kc;
+    a.cw = CTA_INTS;
+    a.cta = m->w_bcta.p;
+    a.sl_ptr = S.sl_ptr.p;
+    a.sl_width = S.sl_width.p;
+    a.col = S.col.p;
+    a.val = mixed ? (const void *)S.v32.p : (const void *)S.v64.p;
+    a.val64 = S.v64.p;
+    a.b = b;
+    a.x = x;
+    a.r = r;
+    a.z = z;
+    a.p = p;
+    a.p2 = p2;
+    a.prec = prec;
+    a.mail = reinterpret_cast<Mail *>(m->w_bmail.p);
+    a.epoch = m->mail_epoch + 1;
+    m->mail_epoch += 4 * (unsigned long long)P.budget;   // an iteration and a replacement: four exchanges at most
+    a.sc = sc;
+    a.rtol = rtol;
+    a.drop2 = drop2;
+    a.maxit = maxit;
+    a.budget = P.budget;
+    const void *fn = S.nd == 3 ? (mixed ? fn_nr<3, float, false>(nr, P.rpt) : fn_nr<3, double, false>(nr, P.rpt))
+                     : blocks2 ? fn_nr<2, float, true>(nr, P.rpt)
+                               : fn_nr<2, double, false>(nr, P.rpt);
+    if (!fn) return fail(OGB_E_STATE, "batched CG iterations: no kernel of this shape");
+    OGB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
+    void *args[] = {&a};
+    const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(P.grid), dim3(P.nt), args, P.smem, s);
+    if (e != cudaSuccess) return cuda_fail(e, "cooperative launch of the batched CG iterations");
+    count_launch(ctx);
+    return OGB_OK;
+}
+
+}  // namespace ogb

@@ -352,3 +352,41 @@ def test_rve_batch_mixed_small_rves_reliable(ctx, native_lib, oracle):
         for lc in range(3):
             ref = _oracle_case(oracle, m, mg.rve_bc_values(m, lc), np.zeros_like(m.bc_value), 1e-13)
             assert rel(u[lc, sl], ref["u"]) < 1e-6, (i, lc)
+
+
+@pytest.mark.parametrize("kind,sides,nrhs", [("rve", (1, 2, 3), 3), ("rve", (8, 40, 9, 17), 4), ("rve", (30,) * 20, 2),
+                                             ("rve", (60, 64, 75), 3), ("rve", (110, 5), 1), ("tet", (3, 8, 5), 1),
+                                             ("tet", (12, 12, 11), 1), ("tet", (6, 9), 2)])
+def test_batch_in_one_launch(kind, sides, nrhs, native_lib):
+    """Batches small enough for one launch (every instance on CTAs of its own,
+    residual replacements inside) against the per-iteration launches, which an
+    option that chooses a form of them keeps: instances of one CTA and of many, one
+    to four node rows per thread and load cases, an instance without a free DOF,
+    two and three DOFs per node, both precisions. Both meet the same tolerance on
+    the FP64 residual (1e-12 and 1e-10), so they differ by it times the condition
+    number (below 1e5 here) at most; the launch is bitwise reproducible."""
+    from oofem_gb300 import meshgen as mg
+    if kind == "rve":
+        meshes = [mg.quad_rve(n, seed=i) for i, n in enumerate(sides)]
+        bc = np.stack([np.concatenate([mg.rve_bc_values(m, c % 3) * (1 + c // 3) for m in meshes]) for c in range(nrhs)])
+    else:
+        meshes = [mg.tet_cube_linear(n, jitter=0.15, seed=i) for i, n in enumerate(sides)]
+        bc = np.stack([np.concatenate([m.bc_value for m in meshes]) * (1 + c) for c in range(nrhs)])
+    big, starts = mg.concat_meshes(meshes)
+    for prec, rtol, tol in ((native_lib.PREC_FP64, 1e-12, 1e-7), (native_lib.PREC_MIXED, 1e-10, 1e-5)):
+        out = []
+        for forced in (False, False, True):
+            c = native_lib.Context(0)
+            if forced:
+                c.set_option(native_lib.OPT_BATCH_X64, 0)
+            model = native_lib.GpuModel(c, big)
+            model.set_instances(starts)
+            A = native_lib.GpuCsrMtrx(c)
+            u, reac, its, ach, st = model.batch_linear_static(A, bc, rtol=rtol, precision=prec)
+            assert (st == 0).all() and (ach <= rtol).all(), (st, ach)
+            out.append((u, reac, its, c.kernel_launches()))
+        a, b, f = out
+        assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1]) and np.array_equal(a[2], b[2])
+        for k in range(nrhs):
+            assert rel(a[0][k], f[0][k]) < tol and rel(a[1][k], f[1][k]) < tol, (rel(a[0][k], f[0][k]), rel(a[1][k], f[1][k]))
+        assert a[3] < f[3]
