@@ -169,6 +169,22 @@ struct HalfSell {
     }
 };
 
+// Coarse part of the mixed preconditioner (coarse.cu): boxes of nodes, their rigid
+// motions, the inverse of the coarse matrix.
+struct Coarse {
+    bool tried = false, ok = false;
+    int nm = 0, nc = 0, ncp = 0, nparts = 0;   // motions per box; coarse equations (padded); CTAs of W^T r
+    DBuf<int> box, list, part, box_part;       // box of a row; rows by box; first row of each part; first part of each box
+    DBuf<int> need;                            // rows that add to the coarse matrix
+    int nlist = 0;
+    DBuf<float> rel;                           // position in the box, planes
+    DBuf<long long> fixed;
+    DBuf<unsigned long long> maxd;
+    DBuf<double> a, b, d, parts, c;
+    const double *inv = nullptr;
+    int64_t version = -1;
+};
+
 struct SellMat {
     int nd = 0;
     int nact = 0;           // active node rows
@@ -189,6 +205,9 @@ struct SellMat {
     int bform32 = 0;        // batched FP32 SpMV form timed for this matrix: 1 plain, 2 values of a group first
     std::vector<int> inst_nact;           // active node rows of each instance
     std::vector<int64_t> inst_row_base;   // first node-space row of each instance (+ total)
+    DBuf<double> xyz;                     // node coordinates of the active rows, planes
+    DBuf<int> free_mask;                  // free DOFs of a row's node
+    Coarse coarse;
     HalfSell half;                        // half-stored FP32 copy (built on first use)
     int64_t nns() const { return (int64_t)nslices * 32 * nd; }
 };
@@ -322,6 +341,8 @@ struct ogb_mtrx {
     ogb::SellMat sell;
     ogb::DBuf<double> n_b, n_x, n_r64, n_q64;   // node-space FP64 vectors
     ogb::DBuf<float> n_d32;                      // mixed: solution increment since the last replacement
+    bool last_coarse = false;                    // the last mixed solve used the coarse part of the preconditioner
+    int64_t coarse_off = -1;                     // matrix version it does not work on
     bool last_half = false;                      // the last mixed solve used the half-stored FP32 copy
     int precond = 1;                             // IML preconditioner type: 0 none, 1 diagonal, 2 ILU, 4 incomplete Cholesky
     ogb::IcFactor ic;
@@ -459,6 +480,13 @@ struct BatchPersistPlan {
 bool batch_persist_plan(const ogb_ctx *ctx, const SellMat &S, int nr, bool mixed, BatchPersistPlan &P);
 int batch_persist_run(ogb_mtrx *m, const BatchPersistPlan &P, int nr, bool mixed, const double *b, double *x, void *r, void *z,
                       void *p, void *p2, const void *prec, bool blocks2, BatchScal *sc, double rtol, int maxit, double drop2);
+
+// coarse.cu: coarse part of the mixed preconditioner.
+constexpr int COARSE_MIN_NODES = 4096;
+bool coarse_wanted(const ogb_ctx *ctx, const SellMat &S);
+int refresh_coarse(ogb_ctx *ctx, SellMat &S, int64_t version);
+int launch_coarse(ogb_ctx *ctx, SellMat &S, const float *r, const float *z, float *p, double *part, unsigned int *count,
+                  PcgScal *sc, int maxit, int replace, int first);
 
 // direct.cu: LDL^T factor of m (cached per version) and x = A^-1 b on padded
 // equation-space device vectors (info: 0 iterations, FP64 relative residual).

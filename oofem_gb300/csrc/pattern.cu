@@ -668,6 +668,22 @@ __global__ void k_ns_of_eq(int nnodes, int ndofpn, const int *eq, const int *act
     }
 }
 
+// Coordinates (planes) and free DOFs of every node row; padding rows: zero, all free
+// (an identity block that no other row refers to).
+__global__ void k_row_geometry(int nrows, int nd, const int *__restrict__ rownode, const double *__restrict__ coords,
+                               const int *__restrict__ eq, double *__restrict__ xyz, int *__restrict__ mask)
+{
+    const int a = blockIdx.x * blockDim.x + threadIdx.x;
+    if (a >= nrows) return;
+    const int A = rownode[a];
+    int f = A < 0 ? (1 << nd) - 1 : 0;
+    for (int d = 0; d < nd; ++d) {
+        xyz[(size_t)d * nrows + a] = A < 0 ? 0.0 : coords[(size_t)A * nd + d];
+        if (A >= 0 && eq[(size_t)A * nd + d] > 0) f |= 1 << d;
+    }
+    mask[a] = f;
+}
+
 }  // namespace
 
 int build_sell(ogb_model *md, ogb_mtrx *m)
@@ -726,7 +742,11 @@ int build_sell(ogb_model *md, ogb_mtrx *m)
     OGB_CHECK(S.sl_ptr.alloc(nslices + 1));
     OGB_CHECK(S.sl_width.alloc(nslices));
     k_slice_width<<<nblk(nslices + 1), NTHREADS, 0, st>>>(nslices, width.p, S.sl_width.p, S.sl_ptr.p);
-    count_launch(ctx, 3);
+    OGB_CHECK(S.xyz.alloc((size_t)nd * nrows_pad));
+    OGB_CHECK(S.free_mask.alloc(nrows_pad));
+    k_row_geometry<<<nblk(nrows_pad), NTHREADS, 0, st>>>(nrows_pad, nd, rownode.p, md->coords.p, md->eq.p, S.xyz.p, S.free_mask.p);
+    S.coarse.tried = S.coarse.ok = false;
+    count_launch(ctx, 4);
     int64_t nslots = 0;
     OGB_CHECK(exclusive_scan_i64(ctx, S.sl_ptr.p, S.sl_ptr.p, nslices + 1, &nslots));
     S.nslots = nslots;

@@ -465,7 +465,7 @@ __host__ __device__ constexpr int sym_plane(int i, int j)
 // Epilogue of the replacement kernels: ||r64||^2, r.z, r.p -> rho, beta, the
 // coefficient of z in the next p update and the end of the new cycle.
 __device__ __forceinline__ void finish_replace(double (&v)[3], double *part, unsigned int *count, PcgScal *sc,
-                                               int first, int orth, int cycle_cap)
+                                               int first, int orth, int cycle_cap, int coarse = 0)
 {
     block_sum<3>(v);
     if (publish_partials<3>(v, part, count)) {
@@ -475,7 +475,9 @@ __device__ __forceinline__ void finish_replace(double (&v)[3], double *part, uns
         *count = 0;
         sc->rmax2 = t[0];
         sc->rnorm2 = t[0];
-        if (!isfinite(t[1]) || !(t[1] > 0.0)) {
+        if (coarse) {   // rho and beta follow with the coarse part of z (k_coarse_solve)
+            sc->rho_old = t[1];
+        } else if (!isfinite(t[1]) || !(t[1] > 0.0)) {
             sc->done = 2;
         } else {
             sc->beta = first ? 0.0 : t[1] / sc->rho;
@@ -521,7 +523,7 @@ __global__ void __launch_bounds__(NTHREADS) k_mixed_replace_bj(int64_t nnodes, c
                                                                float *__restrict__ r, float *__restrict__ z,
                                                                const P *__restrict__ p, const float *__restrict__ binv,
                                                                double *part, unsigned int *count, PcgScal *sc,
-                                                               int first, int orth, int cycle_cap)
+                                                               int first, int orth, int cycle_cap, int coarse)
 {
     double v[3] = {0, 0, 0};
     int64_t lo, hi;
@@ -545,7 +547,7 @@ __global__ void __launch_bounds__(NTHREADS) k_mixed_replace_bj(int64_t nnodes, c
             v[2] += (double)rr[d] * (double)p[a * ND + d];
         }
     }
-    finish_replace(v, part, count, sc, first, orth, cycle_cap);
+    finish_replace(v, part, count, sc, first, orth, cycle_cap, coarse);
 }
 
 // Inverse of every node's ND x ND diagonal block of the FP64 node-block copy
@@ -688,6 +690,8 @@ __device__ __forceinline__ bool publish_after_sum(double (&v)[2], double *part, 
 }
 
 // Run by every thread of the last block; thread 0 writes the scalars.
+// maxit < 0: the coarse part of z is still to come, and with it the decision
+// (k_coarse_solve); r.z of the block Jacobi part waits in rho_old.
 __device__ __forceinline__ void finish_update32_last(double *part, unsigned int *count, PcgScal *sc, int maxit)
 {
     double t[2];
@@ -695,6 +699,10 @@ __device__ __forceinline__ void finish_update32_last(double *part, unsigned int 
     if (threadIdx.x != 0) return;
     *count = 0;
     sc->rnorm2 = t[0];
+    if (maxit < 0) {
+        sc->rho_old = t[1];
+        return;
+    }
     sc->iters += 1;
     if (!isfinite(t[0]) || !isfinite(t[1])) {
         sc->done = 2;
@@ -1889,7 +1897,15 @@ int pcg_mixed_core(ogb_mtrx *m, const Op &op, const double *v64, const float *v3
     // resident blocks per SM (its occupancy, queried once), or the option's count;
     // each block takes an equal contiguous share of the nodes
     // (the fused form is a cooperative launch: at most its occupancy per SM)
-    const bool fuse = ctx->fused_update && op.sell;
+    // (with the coarse part of the preconditioner z is not complete after the update)
+    bool coarse = sizeof(X) == 4 && sizeof(P) == 4 && op.sell && ctx->mixed_bj && m->precond == 1 && ctx->mixed_diff &&
+                  ctx->mixed_x64 && !ctx->mixed_sum32 && !ctx->mixed_orth && m->coarse_off != m->version && coarse_wanted(ctx, *op.S);
+    if (coarse) {
+        OGB_CHECK(refresh_coarse(ctx, const_cast<SellMat &>(*op.S), m->version));
+        coarse = op.S->coarse.ok;
+    }
+    m->last_coarse = coarse;
+    const bool fuse = ctx->fused_update && op.sell && !coarse;
     const void *ufn = op.sell ? bj_update_fn(op.S->nd, ctx->mixed_x64 ? (ctx->mixed_sum32 ? 2 : 1) : (ctx->mixed_sum32 ? 0 : 3), fuse)
                               : nullptr;
     // (at most the occupancy, and no more blocks per SM than give each block about
@@ -1982,7 +1998,7 @@ int pcg_mixed_core(ogb_mtrx *m, const Op &op, const double *v64, const float *v3
     m->last_half = half;
     // small systems: the iterations between two replacements in one launch
     PersistPlan plan;
-    const bool persist = F32 && sizeof(P) == 4 && bj && diff && !half && ctx->mixed_x64 && !ctx->mixed_sum32 &&
+    const bool persist = F32 && sizeof(P) == 4 && bj && diff && !half && !coarse && ctx->mixed_x64 && !ctx->mixed_sum32 &&
                          persist_plan(ctx, *op.S, true, plan);
     if (persist) {
     } else if (half) {
@@ -2021,8 +2037,13 @@ int pcg_mixed_core(ogb_mtrx *m, const Op &op, const double *v64, const float *v3
                 if (bj) {
                     void *xs = ctx->mixed_x64 ? (void *)x : (void *)d;
                     OGB_CHECK(launch_bj_update(ufn, fuse, gu, zbytes, s, nnodes, xs, r, z, p, q, binv, m->w_part.p,
-                                               m->w_count.p, m->w_epoch.p, zcap, sc, maxit));
-                    if (!fuse) k_pupdate_f32<<<gu, NTHREADS, 0, s>>>(op.n, z, p, sc);
+                                               m->w_count.p, m->w_epoch.p, zcap, sc, coarse ? -1 : maxit));
+                    if constexpr (F32 && sizeof(P) == 4) {
+                        if (coarse)
+                            OGB_CHECK(launch_coarse(ctx, const_cast<SellMat &>(*op.S), r, z, p, m->w_part.p, m->w_count.p, sc,
+                                                    maxit, 0, 0));
+                    }
+                    if (!fuse && !coarse) k_pupdate_f32<<<gu, NTHREADS, 0, s>>>(op.n, z, p, sc);
                 } else if (ctx->mixed_x64) {
                     k_update_rz32<<<gb, NTHREADS, 0, s>>>(op.n, x, r, z, p, q, dinv, m->w_part.p, m->w_count.p, sc,
                                                            maxit);
@@ -2037,7 +2058,7 @@ int pcg_mixed_core(ogb_mtrx *m, const Op &op, const double *v64, const float *v3
                                                           rtol, maxit);
                 k_pupdate4<P><<<gb, NTHREADS, 0, s>>>(op.n, z, p, sc);
             }
-            count_launch(ctx, bj && fuse ? 1 : 2);
+            count_launch(ctx, coarse || (bj && fuse) ? 1 : 2);
         }
         if constexpr (F32) {
             if (!ctx->mixed_x64) {
@@ -2073,7 +2094,7 @@ int pcg_mixed_core(ogb_mtrx *m, const Op &op, const double *v64, const float *v3
         // (six replacement cycles without halving it, or a breakdown of the
         // FP32 recurrences); the caller finishes the solve in FP64
         if (!(achieved < 0.5 * mark)) {
-            if (++since_mark >= 6 || replacements > 400) {
+            if (++since_mark >= (coarse ? 2 : 6) || replacements > 400) {
                 *stalled = true;
                 break;
             }
@@ -2089,24 +2110,31 @@ int pcg_mixed_core(ogb_mtrx *m, const Op &op, const double *v64, const float *v3
         }
         // replacement: r = r64, z = D^-1 r, beta; then p = z + beta p
         // cycle cap: unbounded for the first cycle, then twice the longest cycle so far (at least 512)
-        const int cap = first ? (maxit < (1 << 29) ? maxit : (1 << 29)) : (2 * longest > 512 ? 2 * longest : 512);
+        // (with the coarse part a cycle is a few dozen iterations; one that is not has an
+        // operator beyond FP32, and the solve goes on without it)
+        const int cap = coarse ? std::min(maxit, iters + 512) - iters : first ? (maxit < (1 << 29) ? maxit : (1 << 29)) : (2 * longest > 512 ? 2 * longest : 512);
         if constexpr (F32) {
             if (bj) {
                 if (nd == 3)
                     k_mixed_replace_bj<3, P><<<g, NTHREADS, 0, s>>>(nnodes, r64, r, z, p, binv, m->w_part.p,
                                                                      m->w_count.p, sc, first ? 1 : 0,
-                                                                     ctx->mixed_orth ? 1 : 0, cap);
+                                                                     ctx->mixed_orth ? 1 : 0, cap, coarse ? 1 : 0);
                 else
                     k_mixed_replace_bj<2, P><<<g, NTHREADS, 0, s>>>(nnodes, r64, r, z, p, binv, m->w_part.p,
                                                                      m->w_count.p, sc, first ? 1 : 0,
-                                                                     ctx->mixed_orth ? 1 : 0, cap);
+                                                                     ctx->mixed_orth ? 1 : 0, cap, coarse ? 1 : 0);
             }
         }
         if (!bj)
             k_mixed_replace<X, P><<<g, NTHREADS, 0, s>>>(nch, r64, r, z, p, dinv, m->w_part.p, m->w_count.p, sc,
                                                          first ? 1 : 0, ctx->mixed_orth ? 1 : 0, cap);
-        k_pcg_pupdate<X, P><<<g, NTHREADS, 0, s>>>(n, z, p, sc);
-        count_launch(ctx, 2);
+        if constexpr (F32 && sizeof(P) == 4) {
+            if (coarse)
+                OGB_CHECK(launch_coarse(ctx, const_cast<SellMat &>(*op.S), r, z, p, m->w_part.p, m->w_count.p, sc, maxit, 1,
+                                        first ? 1 : 0));
+        }
+        if (!coarse) k_pcg_pupdate<X, P><<<g, NTHREADS, 0, s>>>(n, z, p, sc);
+        count_launch(ctx, coarse ? 1 : 2);
         first = false;
         ++replacements;
         // iterations on the FP32 operator until the next replacement is due
@@ -2118,7 +2146,7 @@ int pcg_mixed_core(ogb_mtrx *m, const Op &op, const double *v64, const float *v3
                 OGB_CHECK(persist_run(m, plan, true, v32, x, r, p, z, q, binv, rtol, maxit));
             } else if (ctx->use_graphs) {
                 OGB_CHECK(graph.launch(ctx));
-                count_launch(ctx, (bj && fuse ? 2 : 3) * BATCH + (F32 && !ctx->mixed_x64 ? 1 : 0));
+                count_launch(ctx, (coarse ? 5 : bj && fuse ? 2 : 3) * BATCH + (F32 && !ctx->mixed_x64 ? 1 : 0));
             } else {
                 OGB_CHECK(batch());
             }
@@ -2278,9 +2306,16 @@ int pcg_mixed(ogb_mtrx *m, const double *b, double *x, double rtol, int maxit, o
     OGB_CHECK(to_op_space(m, op, b, x, &bo, &xo));
     ogb_solve_info mi{};
     bool stalled = false;
-    if (m->ctx->mixed_vec32)
+    if (m->ctx->mixed_vec32) {
         OGB_CHECK((pcg_mixed_core<float, float>(m, op, v64, v32, bo, xo, rtol, maxit, &mi, &stalled)));
-    else if (m->ctx->mixed_p32)
+        if (stalled && mi.status != OGB_OK && m->last_coarse && mi.iterations < maxit) {
+            // stiffnesses too far apart for the coarse matrix: go on without it
+            const int done = mi.iterations;
+            m->coarse_off = m->version;
+            OGB_CHECK((pcg_mixed_core<float, float>(m, op, v64, v32, bo, xo, rtol, maxit - done, &mi, &stalled)));
+            mi.iterations += done;
+        }
+    } else if (m->ctx->mixed_p32)
         OGB_CHECK((pcg_mixed_core<double, float>(m, op, v64, v32, bo, xo, rtol, maxit, &mi, &stalled)));
     else
         OGB_CHECK((pcg_mixed_core<double, double>(m, op, v64, v32, bo, xo, rtol, maxit, &mi, &stalled)));

@@ -538,7 +538,8 @@ def test_one_launch_iterations(mesh, size, native_lib):
         a, b, f = out
         assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1]) and a[2] == b[2]
         assert rel(a[0], f[0]) < tol and rel(a[1], f[1]) < tol, (rel(a[0], f[0]), rel(a[1], f[1]))
-        assert a[3] < f[3] or f[2] < 8
+        # (mixed solves from 4,096 nodes on take the coarse preconditioner's launches)
+        assert a[3] < f[3] or f[2] < 8 or (prec == native_lib.PREC_MIXED and m.nnodes > 4096)
     # the iteration limit holds as before
     _, _, info = model.linear_static(A, rtol=1e-30, maxit=5)
     c = native_lib.Context(0)
@@ -546,3 +547,35 @@ def test_one_launch_iterations(mesh, size, native_lib):
     A = native_lib.GpuCsrMtrx(c)
     _, _, one = model.linear_static(A, rtol=1e-30, maxit=5)
     assert one.iterations == info.iterations and one.status == info.status
+
+
+@pytest.mark.parametrize("mesh,size", [("hex", (40, 11, 9)), ("hex", (90, 6, 6)), ("hex", (101, 21, 19)), ("quad", 66),
+                                       ("quad", 200), ("tet", 17), ("tet", 30)])
+def test_coarse_preconditioner(mesh, size, native_lib):
+    """Mixed solves with the coarse part of the preconditioner (from 4,096 active
+    nodes on): the residual tolerance is met, the solution is that of the FP64 solve
+    to the tolerances times the condition number (below 1e5; 1e-10 and 1e-12), the
+    result is bitwise reproducible, and the iterations are fewer than block Jacobi's
+    alone (kept by contexts that choose a form of the launches)."""
+    from oofem_gb300 import meshgen as mg
+    m = mg.hex_cantilever(*size, jitter=0.2, seed=3) if mesh == "hex" else \
+        mg.quad_rve(size, seed=3) if mesh == "quad" else mg.tet_cube_linear(size, jitter=0.15, seed=3)
+    model = native_lib.GpuModel(native_lib.Context(0), m)
+    ref, rref, _ = model.linear_static(native_lib.GpuCsrMtrx(model.ctx), rtol=1e-12)
+    out = []
+    for forced in (False, False, True):
+        c = native_lib.Context(0)
+        if forced:
+            c.set_option(native_lib.OPT_FUSED_UPDATE, 1)
+        model = native_lib.GpuModel(c, m)
+        A = native_lib.GpuCsrMtrx(c)
+        u, reac, info = model.linear_static(A, rtol=1e-10, maxit=100000, precision=native_lib.PREC_MIXED)
+        assert info.status == 0 and info.achieved <= 1e-10 and A.last_block_jacobi()
+        assert rel(u, ref) < 1e-6 and rel(reac, rref) < 1e-6, (rel(u, ref), rel(reac, rref))
+        # the matrix's second values: the coarse matrix follows them
+        u2, _, i2 = model.linear_static(A, rtol=1e-10, maxit=100000, precision=native_lib.PREC_MIXED)
+        assert np.array_equal(u, u2) and info.iterations == i2.iterations
+        out.append((u, info.iterations))
+    assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]
+    assert out[0][1] < out[2][1], (out[0][1], out[2][1])
+    print(mesh, size, "iterations", out[0][1], "without", out[2][1])
