@@ -60,7 +60,8 @@ __device__ __forceinline__ bool publish_inst(const double (&v)[NV], double *part
 }
 
 // Fixed-order sums of the partials of units [u0, u1), one value per warp (see
-// block_sum for why); returned in shared memory, for every thread.
+// block_sum for why); returned in shared memory, for every thread. Lane l of chunk w
+// takes units u0 + 32 w + l, + 256, ..., the chunks' lane sums are added in order.
 template <int NV>
 __device__ __forceinline__ const double *inst_sums(const double *part, int64_t u0, int64_t u1)
 {
@@ -68,11 +69,14 @@ __device__ __forceinline__ const double *inst_sums(const double *part, int64_t u
     const int lane = threadIdx.x & 31;
     __threadfence();
     for (int k = threadIdx.x >> 5; k < NV; k += NTHREADS / 32) {
-        double s = 0.0;
+        double sum = 0.0;
+        for (int w = 0; w < NTHREADS / 32 && u0 + 32 * w < u1; ++w) {
+            double s = 0.0;
 #pragma unroll 4
-        for (int64_t u = u0 + lane; u < u1; u += 32) s += __ldcg(part + u * NV + k);
-        s = warp_sum(s);
-        if (lane == 0) tot[k] = s;
+            for (int64_t u = u0 + 32 * w + lane; u < u1; u += NTHREADS) s += __ldcg(part + u * NV + k);
+            sum += warp_sum(s);
+        }
+        if (lane == 0) tot[k] = sum;
     }
     __syncthreads();
     return tot;
@@ -488,7 +492,7 @@ __global__ void __launch_bounds__(NTHREADS) k_breplace(const double *__restrict_
                                                        float *__restrict__ z, double *part, unsigned int *cnt,
                                                        BatchScal *sc, const int *__restrict__ unit_inst,
                                                        const int64_t *__restrict__ unit_ptr, double rtol, int maxit,
-                                                       int init)
+                                                       int init, int coarse)
 {
     const int inst = unit_inst[blockIdx.x];
     if (inst_skip<NR>(sc, inst, init ? 2 : 3)) return;
@@ -521,7 +525,7 @@ __global__ void __launch_bounds__(NTHREADS) k_breplace(const double *__restrict_
         }
     }
     const int64_t u0 = unit_ptr[inst], u1 = unit_ptr[inst + 1];
-    block_sum<3 * NR>(v);
+    block_sum_shuffle<3 * NR>(v);
     if (!publish_inst<3 * NR>(v, part, blockIdx.x, cnt + inst, u1 - u0)) return;
     const double *t = inst_sums<3 * NR>(part, u0, u1);
     if (threadIdx.x == 0) cnt[inst] = 0;
@@ -552,7 +556,10 @@ __global__ void __launch_bounds__(NTHREADS) k_breplace(const double *__restrict_
         if (sqrt(t[NR + c]) / normb <= rtol) s.done = 1;
         else if (!isfinite(t[NR + c])) s.done = 2;
         else if (s.iters >= maxit) s.done = 4;
-        else if (!isfinite(rz) || !(rz > 0.0) || s.since >= 6) s.done = 5;
+        else if (coarse) {   // the coarse part of z is still to come (k_bcoarse_solve)
+            s.rz1 = rz;
+            s.repl = 2;
+        } else if (!isfinite(rz) || !(rz > 0.0) || s.since >= 6) s.done = 5;
         else {
             s.beta = init ? 0.0 : rz / s.rho;
             s.rho = rz;
@@ -618,6 +625,10 @@ __global__ void __launch_bounds__(NTHREADS) k_bupdate32(XS *__restrict__ x, floa
         BatchScal &s = sc[inst * NR + c];
         if (!pair_running<NR>(s)) return;
         s.rnorm2 = t[c];
+        if (drop2 < 0.0) {   // the coarse part of z is still to come, and with it the decision (k_bcoarse_solve)
+            s.rz1 = t[NR + c];
+            return;
+        }
         s.iters += 1;
         s.repl = 0;
         double normb = sqrt(s.bnorm2);
@@ -704,7 +715,7 @@ struct BatchWork {
     DBuf<int> vinst, sinst, zero;
     DBuf<int64_t> vptr, sptr;
     DBuf<BatchScal> sc;
-    DBuf<double> part, r, z, p, q, dinv, q64;
+    DBuf<double> part, r, z, p, q, dinv, q64, cpart;
     DBuf<float> r32, z32, p32, q32, dinv32;
     DBuf<float2> binv2;   // block Jacobi rows (two DOFs per node)
     DBuf<float> d32;      // FP32 solution increment of the current batch (batch_x64 off)
@@ -738,7 +749,7 @@ struct ExecGuard {
 };
 
 template <int ND, int NR>
-int run_batch(ogb_mtrx *m, const double *b, double *x, double rtol, int maxit, bool mixed,
+int run_batch(ogb_mtrx *m, const double *b, double *x, const double rtol_asked, int maxit, bool mixed,
               std::vector<BatchScal> &res)
 {
     ogb_ctx *ctx = m->ctx;
@@ -802,6 +813,17 @@ int run_batch(ogb_mtrx *m, const double *b, double *x, double rtol, int maxit, b
     // small batches: every instance's iterations (and its residual replacements) in one launch
     BatchPersistPlan plan;
     const bool persist = batch_persist_plan(ctx, S, NR, mixed, plan);
+    // larger ones, mixed: coarse part of the preconditioner (coarse.cu)
+    bool coarse = mixed && !persist && batch_coarse_wanted(ctx, S, rtol_asked);
+    if (coarse) {
+        OGB_CHECK(refresh_coarse(ctx, m->sell, m->version));
+        coarse = S.coarse.ok;
+    }
+    if (coarse) OGB_CHECK(w.cpart.alloc((size_t)ninst * S.coarse.maxblocks * 4 * NR));
+    const double drop2c = ctx->mixed_drop * ctx->mixed_drop, rtol = coarse ? COARSE_MARGIN * rtol_asked : rtol_asked;
+    auto coarse_step = [&](int mode) {
+        return launch_batch_coarse(ctx, m->sell, NR, w.r32.p, w.z32.p, w.p32.p, w.cpart.p, w.cnt.p, w.sc.p, rtol, drop2c, maxit, mode);
+    };
     // mixed preconditioner: FP32 block Jacobi of the 2 x 2 node blocks (two DOFs
     // per node) where the option allows it, else the scalar diagonal
     const bool bj2 = mixed && ND == 2 && ctx->mixed_bj;
@@ -809,10 +831,10 @@ int run_batch(ogb_mtrx *m, const double *b, double *x, double rtol, int maxit, b
         if (bj2)
             k_breplace<NR, true><<<nvu, NTHREADS, 0, st>>>(b, w.q64.p, w.dinv32.p, w.binv2.p, w.r32.p, w.z32.p,
                                                            w.part.p, w.cnt.p, w.sc.p, w.vinst.p, w.vptr.p, rtol, maxit,
-                                                           init);
+                                                           init, coarse ? 1 : 0);
         else
             k_breplace<NR><<<nvu, NTHREADS, 0, st>>>(b, w.q64.p, w.dinv32.p, nullptr, w.r32.p, w.z32.p, w.part.p,
-                                                     w.cnt.p, w.sc.p, w.vinst.p, w.vptr.p, rtol, maxit, init);
+                                                     w.cnt.p, w.sc.p, w.vinst.p, w.vptr.p, rtol, maxit, init, coarse ? 1 : 0);
     };
     if (mixed) {
         m->last_bj = bj2;
@@ -826,9 +848,10 @@ int run_batch(ogb_mtrx *m, const double *b, double *x, double rtol, int maxit, b
         // p starts at zero: the init pass's p = z + 0 p is z
         OGB_CUDA(cudaMemsetAsync(w.p32.p, 0, nv * sizeof(float), st));
         replace(1);
-        k_bpupdate32<NR><<<nvu, NTHREADS, 0, st>>>(w.z32.p, w.p32.p, w.sc.p, w.vinst.p, 1);
+        if (coarse) OGB_CHECK(coarse_step(2));
+        else k_bpupdate32<NR><<<nvu, NTHREADS, 0, st>>>(w.z32.p, w.p32.p, w.sc.p, w.vinst.p, 1);
         const bool diff = ctx->mixed_diff;
-        const double drop2 = ctx->mixed_drop * ctx->mixed_drop;
+        const double drop2 = coarse ? -1.0 : ctx->mixed_drop * ctx->mixed_drop;
         // one iteration: q = K p (FP32), the updates (pairs whose recursive residual
         // dropped by the drop factor pause), p = z + beta p for the running pairs
         // FP32 SpMV form, timed once per matrix (the launches recompute q, p.q and
@@ -919,7 +942,8 @@ int run_batch(ogb_mtrx *m, const double *b, double *x, double rtol, int maxit, b
                 k_bupdate32<NR, false, float><<<nvu, NTHREADS, 0, st>>>(w.d32.p, w.r32.p, w.z32.p, w.p32.p, w.q32.p,
                                                                         w.dinv32.p, nullptr, w.part.p, w.cnt.p, w.sc.p,
                                                                         w.vinst.p, w.vptr.p, rtol, maxit, drop2);
-            k_bpupdate32<NR><<<nvu, NTHREADS, 0, st>>>(w.z32.p, w.p32.p, w.sc.p, w.vinst.p, 0);
+            if (coarse) coarse_step(0);
+            else k_bpupdate32<NR><<<nvu, NTHREADS, 0, st>>>(w.z32.p, w.p32.p, w.sc.p, w.vinst.p, 0);
             if (!x64 && ++*calls % BBATCH == 0) k_bfold<<<num_sms() * 4, NTHREADS, 0, st>>>(nv, x, w.d32.p);
         };
     } else {
@@ -974,8 +998,9 @@ int run_batch(ogb_mtrx *m, const double *b, double *x, double rtol, int maxit, b
             // beta, and their p = z + beta p
             residual_spmv(w.q64.p, 3);
             replace(0);
-            k_bpupdate32<NR><<<nvu, NTHREADS, 0, st>>>(w.z32.p, w.p32.p, w.sc.p, w.vinst.p, 1);
-            count_launch(ctx, 3);
+            if (coarse) OGB_CHECK(coarse_step(1));
+            else k_bpupdate32<NR><<<nvu, NTHREADS, 0, st>>>(w.z32.p, w.p32.p, w.sc.p, w.vinst.p, 1);
+            count_launch(ctx, coarse ? 5 : 3);
             OGB_CUDA(cudaGetLastError());
             continue;
         }
@@ -984,7 +1009,7 @@ int run_batch(ogb_mtrx *m, const double *b, double *x, double rtol, int maxit, b
         } else {
             for (int k = 0; k < BBATCH; ++k) iteration();
         }
-        count_launch(ctx, 3 * BBATCH + (mixed && !ctx->batch_x64 ? 1 : 0));
+        count_launch(ctx, (coarse ? 5 : 3) * BBATCH + (mixed && !ctx->batch_x64 ? 1 : 0));
         OGB_CUDA(cudaGetLastError());
         it += BBATCH;
     }

@@ -10,7 +10,7 @@
 // on the FP64 residual stay as they are; only the search directions are better.
 // Iterations without -> with it, and the solve with set-up (GB300): 290 x 58 x 58 hexes
 // to 1e-8 3,300 -> 350, 660 -> 112 ms; 101 x 21 x 19 to 1e-9 1,760 -> 150, 31 (one launch)
-// -> 9.6 ms; 40^3-cell tets to 1e-11 710 -> 140, 24.6 -> 11.5 ms.
+// -> 10 ms; 40^3-cell tets to 1e-10 about 650 -> 130.
 //
 // Everything is deterministic: Ac is summed in 64-bit integers (fixed point scaled by
 // K's largest diagonal entry), so the order of the atomic additions does not matter;
@@ -27,6 +27,7 @@ namespace ogb {
 namespace {
 
 constexpr int GJ = 32;             // block of the inversion
+constexpr int PADDING = 8;         // free_mask of a padding row
 constexpr double COARSE_SOFTEST = 3e-7;
 constexpr int AC_BITS = 42;        // fixed point of Ac: 2^42 per largest diagonal entry of K (2^18 terms an entry fit)
 
@@ -87,28 +88,28 @@ __global__ void k_max_diag(int nact, const int64_t *__restrict__ diag, const dou
 // Rows that add to Ac: a row whose neighbours all lie in its own box with all DOFs
 // free adds nothing (K times a rigid motion is zero there). About a fifth of a large
 // mesh is left; the list of them keeps warps full of rows that have work.
-__global__ void k_coarse_need(int nact, const int64_t *__restrict__ sl_ptr, const int *__restrict__ sl_width,
+__global__ void k_coarse_need(int nact, const int *__restrict__ rows, const int64_t *__restrict__ sl_ptr, const int *__restrict__ sl_width,
                               const int *__restrict__ col, const int *__restrict__ box, const int *__restrict__ mask, int full,
                               int64_t *__restrict__ flag)
 {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a > nact) return;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t > nact) return;
     bool need = false;
-    if (a < nact) {
-        const int s = a >> 5, r = a & 31, w = sl_width[s], I = box[a];
+    if (t < nact) {
+        const int a = rows[t], s = a >> 5, r = a & 31, w = sl_width[s], I = box[a];
         const int64_t base = sl_ptr[s];
         for (int k = 0; k < w && !need; ++k) {
             const int B = col[base + 32 * k + r];
             need = box[B] != I || mask[B] != full;
         }
     }
-    flag[a] = need ? 1 : 0;
+    flag[t] = need ? 1 : 0;
 }
 
-__global__ void k_coarse_list(int nact, const int64_t *__restrict__ pos, int *__restrict__ list)
+__global__ void k_coarse_list(int nact, const int *__restrict__ rows, const int64_t *__restrict__ pos, int *__restrict__ list)
 {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a < nact && pos[a + 1] > pos[a]) list[pos[a]] = a;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < nact && pos[t + 1] > pos[t]) list[pos[t]] = rows[t];
 }
 
 // Ac += W_a^T K_aB W_B over the blocks of row a, a thread per listed row. The blocks
@@ -120,8 +121,9 @@ __global__ void __launch_bounds__(128) k_coarse_matrix(int nlist, const int *__r
                                                        const int *__restrict__ sl_width, const int *__restrict__ col,
                                                        const double *__restrict__ val, const int *__restrict__ box,
                                                        const float *__restrict__ rel, const int *__restrict__ mask,
-                                                       int64_t nrows, int nc, const unsigned long long *__restrict__ maxd,
-                                                       unsigned long long *A)
+                                                       int64_t nrows, const int *__restrict__ box_inst, const int *__restrict__ box_row,
+                                                       const int *__restrict__ inst, const int64_t *__restrict__ inst_mat,
+                                                       const unsigned long long *__restrict__ maxd, unsigned long long *F)
 {
     constexpr int NM = Modes<ND>::NM;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -138,6 +140,8 @@ __global__ void __launch_bounds__(128) k_coarse_matrix(int nlist, const int *__r
         for (int d = 0; d < ND; ++d) xa[d] = xf[d];
         rigid<ND, double>(xa, mask[a], wa);
     }
+    const int nc = inst[5 * box_inst[I] + 1];
+    unsigned long long *A = F + inst_mat[box_inst[I]] + (size_t)box_row[I] * nc;
     int J = I;   // own box first, then the others in increasing order
     for (;;) {
         double T[ND][NM];
@@ -175,6 +179,7 @@ __global__ void __launch_bounds__(128) k_coarse_matrix(int nlist, const int *__r
                 }
             }
         }
+        const int jc = box_row[J];
 #pragma unroll
         for (int m = 0; m < NM; ++m)
 #pragma unroll
@@ -187,7 +192,7 @@ __global__ void __launch_bounds__(128) k_coarse_matrix(int nlist, const int *__r
                     for (int d = 0; d < ND; ++d) c = fma(wa[d][m], T[d][n], c);
                 }
                 const long long f = __double2ll_rn(c * scale);
-                if (f) atomicAdd(A + (size_t)(I * NM + m) * nc + J * NM + n, (unsigned long long)f);
+                if (f) atomicAdd(A + (size_t)m * nc + jc + n, (unsigned long long)f);
             }
         if (next == 0x7fffffff) break;
         J = next;
@@ -197,19 +202,22 @@ __global__ void __launch_bounds__(128) k_coarse_matrix(int nlist, const int *__r
 // Ac in FP64 on whole blocks of GJ, symmetric; motions no DOF takes part in (a box of
 // one node has no rotations) get a unit diagonal, and a shift of 1e-8 keeps boxes
 // with dependent motions (nodes on a line) positive definite.
-__global__ void k_coarse_convert(int nc, int ncp, const long long *__restrict__ F, const unsigned long long *__restrict__ maxd,
-                                 double *__restrict__ A)
+__global__ void k_coarse_convert(const int *__restrict__ inst, const int64_t *__restrict__ inst_mat, const long long *__restrict__ F0,
+                                 const unsigned long long *__restrict__ maxd, double *__restrict__ A0)
 {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (int64_t)ncp * ncp) return;
-    const int i = (int)(t / ncp), j = (int)(t % ncp);
-    double v = i == j ? 1.0 : 0.0;
-    if (i < nc && j < nc) {
-        const double unit = __longlong_as_double((long long)*maxd) * ldexp(1.0, -AC_BITS);
-        v = 0.5 * ((double)F[(size_t)i * nc + j] + (double)F[(size_t)j * nc + i]) * unit;
-        if (i == j) v = v > 0.0 ? v * (1.0 + 1e-8) : 1.0;
+    const int nc = inst[5 * blockIdx.y], ncp = inst[5 * blockIdx.y + 1];
+    const long long *F = F0 + inst_mat[blockIdx.y];
+    double *A = A0 + inst_mat[blockIdx.y];
+    const double unit = __longlong_as_double((long long)*maxd) * ldexp(1.0, -AC_BITS);
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < (int64_t)ncp * ncp; t += (int64_t)gridDim.x * blockDim.x) {
+        const int i = (int)(t / ncp), j = (int)(t % ncp);
+        double v = i == j ? 1.0 : 0.0;
+        if (i < nc && j < nc) {
+            v = 0.5 * ((double)F[t] + (double)F[(size_t)j * ncp + i]) * unit;
+            if (i == j) v = v > 0.0 ? v * (1.0 + 1e-8) : 1.0;
+        }
+        A[t] = v;
     }
-    A[t] = v;
 }
 
 // Block Gauss-Jordan inversion, step k: D = inverse of the diagonal block (one CTA),
@@ -218,8 +226,13 @@ __global__ void k_coarse_convert(int nc, int ncp, const long long *__restrict__ 
 // In the diagonal step a warp holds rows warp + 8 q and the pivot's owner publishes its
 // scaled row, as in the direct solver's diagonal block (with a division in each of 32
 // warps the step took 76 us).
-__global__ void __launch_bounds__(NTHREADS) k_gj_diag(int n, int k, const double *__restrict__ A, double *__restrict__ D)
+__global__ void __launch_bounds__(NTHREADS) k_gj_diag(const int *__restrict__ inst, const int64_t *__restrict__ inst_mat, int k,
+                                                      const double *__restrict__ A0, double *__restrict__ D0)
 {
+    const int n = inst[5 * blockIdx.x + 1];
+    if (k * GJ >= n) return;
+    const double *A = A0 + inst_mat[blockIdx.x];
+    double *D = D0 + (size_t)blockIdx.x * GJ * GJ;
     __shared__ double W[2][GJ];
     const int c = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double e[4];
@@ -251,9 +264,14 @@ __global__ void __launch_bounds__(NTHREADS) k_gj_diag(int n, int k, const double
     for (int q = 0; q < 4; ++q) D[(warp + 8 * q) * GJ + c] = e[q];
 }
 
-__global__ void __launch_bounds__(NTHREADS) k_gj_update(int n, int k, const double *__restrict__ A, const double *__restrict__ D,
-                                                        double *__restrict__ B)
+__global__ void __launch_bounds__(NTHREADS) k_gj_update(const int *__restrict__ inst, const int64_t *__restrict__ inst_mat, int k,
+                                                        const double *__restrict__ A0, const double *__restrict__ D0,
+                                                        double *__restrict__ B0)
 {
+    const int n = inst[5 * blockIdx.z + 1];
+    if (k * GJ >= n || (int)blockIdx.x * GJ >= n || (int)blockIdx.y * GJ >= n) return;
+    const double *A = A0 + inst_mat[blockIdx.z], *D = D0 + (size_t)blockIdx.z * GJ * GJ;
+    double *B = B0 + inst_mat[blockIdx.z];
     __shared__ double L[GJ][GJ + 1], R[GJ][GJ + 1], M[GJ][GJ + 1];
     const int i = blockIdx.y, j = blockIdx.x, c = threadIdx.x & 31, r0 = threadIdx.x >> 5;
     for (int r = r0; r < GJ; r += 8) {
@@ -289,6 +307,17 @@ __global__ void __launch_bounds__(NTHREADS) k_gj_update(int n, int k, const doub
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) B[(size_t)(i * GJ + r0 + 8 * q) * n + j * GJ + c] = p[q];
+}
+
+// FP32 copy of the inverses, for batches: FP64 products and lane sums of every row by
+// three load cases took 28.6 us an iteration over 64 RVEs.
+__global__ void k_coarse_inv32(const int *__restrict__ inst, const int64_t *__restrict__ inst_mat, const double *__restrict__ a,
+                               const double *__restrict__ b, float *__restrict__ inv32)
+{
+    const int64_t ncp = inst[5 * blockIdx.y + 1], off = inst_mat[blockIdx.y];
+    const double *src = ((ncp / GJ) & 1 ? b : a) + off;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < ncp * ncp; t += (int64_t)gridDim.x * blockDim.x)
+        inv32[off + t] = (float)src[t];
 }
 
 // Partial sums of W^T r: CTA u sums the rows list[first .. last) of one box; a
@@ -387,6 +416,195 @@ __global__ void __launch_bounds__(NTHREADS) k_coarse_solve(int nc, int ncp, int 
     }
 }
 
+// The same for the load cases of a batch, a warp per part: its boxes have a few hundred
+// rows, and a CTA each spent its time in the block sums (16.9 us over 64 RVEs x 3).
+template <int ND, int NR>
+__global__ void __launch_bounds__(NTHREADS) k_bcoarse_restrict(int nparts, const int *__restrict__ part, const int *__restrict__ list,
+                                                               const int *__restrict__ box, const int *__restrict__ box_inst,
+                                                               const float *__restrict__ rel, const int *__restrict__ mask,
+                                                               int64_t nrows, const float *__restrict__ r,
+                                                               float *__restrict__ out, const BatchScal *sc, int mode)
+{
+    constexpr int NM = Modes<ND>::NM;
+    const int u = blockIdx.x * (NTHREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (u >= nparts) return;
+    const int lo = part[u], hi = part[u + 1], inst = box_inst[box[list[lo]]];
+    bool any = false;
+#pragma unroll
+    for (int c = 0; c < NR; ++c) {
+        const BatchScal &q = sc[inst * NR + c];
+        any |= q.done == 0 && (mode ? q.repl == 2 : q.pause == 0);
+    }
+    if (!any) return;
+    float v[NM * NR];
+#pragma unroll
+    for (int m = 0; m < NM * NR; ++m) v[m] = 0.f;
+#pragma unroll 2
+    for (int k = lo + lane; k < hi; k += 32) {
+        const int64_t a = list[k];
+        float x[ND], w[ND][NM];
+        load_rel<ND>(rel, nrows, a, x);
+        rigid<ND, float>(x, mask[a], w);
+#pragma unroll
+        for (int d = 0; d < ND; ++d)
+#pragma unroll
+            for (int c = 0; c < NR; ++c) {
+                const float rd = r[(a * ND + d) * NR + c];
+#pragma unroll
+                for (int m = 0; m < NM; ++m) v[m * NR + c] = fmaf(w[d][m], rd, v[m * NR + c]);
+            }
+    }
+#pragma unroll
+    for (int m = 0; m < NM * NR; ++m) {
+        const float t = warp_sum(v[m]);
+        if (lane == 0) out[(size_t)u * NM * NR + m] = t;
+    }
+}
+
+// c = Ac^-1 w of instance blockIdx.y and, in its last block, its pairs' scalars: the
+// decisions of k_bupdate32 (mode 0) and k_breplace (1; 2 at the start).
+template <int NR>
+__global__ void __launch_bounds__(NTHREADS) k_bcoarse_solve(const int *__restrict__ inst_tab, const int64_t *__restrict__ inst_mat,
+                                                            int nm, const int *__restrict__ box_part,
+                                                            const float *__restrict__ parts, const float *__restrict__ inv32,
+                                                            float *__restrict__ cvec,
+                                                            double *part, unsigned int *cnt, BatchScal *sc, double rtol,
+                                                            double drop2, int maxit, int mode)
+{
+    extern __shared__ float wf[];   // [ncp][NR]
+    const int inst = blockIdx.y, *tab = inst_tab + 5 * inst, nc = tab[0], ncp = tab[1];
+    const int blocks = max(1, (nc + NTHREADS / 32 - 1) / (NTHREADS / 32));
+    if ((int)blockIdx.x >= blocks) return;
+    bool any = false;
+#pragma unroll
+    for (int c = 0; c < NR; ++c) {
+        const BatchScal &q = sc[inst * NR + c];
+        any |= q.done == 0 && (mode ? q.repl == 2 : q.pause == 0);
+    }
+    if (!any) return;
+    for (int i = threadIdx.x; i < ncp * NR; i += NTHREADS) {
+        const int j = i / NR, c = i % NR;
+        float s = 0.f;
+        if (j < nc) {
+            const int b = tab[3] + j / nm, m = j % nm;
+            for (int u = box_part[b]; u < box_part[b + 1]; ++u) s += parts[((size_t)u * nm + m) * NR + c];
+        }
+        wf[i] = s;
+    }
+    __syncthreads();
+    const float *inv = inv32 + inst_mat[inst];
+    const int lane = threadIdx.x & 31, row = blockIdx.x * (NTHREADS / 32) + (threadIdx.x >> 5);
+    double v[NR];
+#pragma unroll
+    for (int c = 0; c < NR; ++c) v[c] = 0.0;
+    if (row < nc) {
+        const float *q = inv + (size_t)row * ncp;
+        float s[NR];
+#pragma unroll
+        for (int c = 0; c < NR; ++c) s[c] = 0.f;
+#pragma unroll 4
+        for (int j = lane; j < ncp; j += 32) {
+            const float a = __ldg(q + j);
+#pragma unroll
+            for (int c = 0; c < NR; ++c) s[c] = fmaf(a, wf[j * NR + c], s[c]);
+        }
+#pragma unroll
+        for (int c = 0; c < NR; ++c) {
+            s[c] = warp_sum(s[c]);
+            if (lane == 0) {
+                cvec[(size_t)(tab[2] + row) * NR + c] = s[c];
+                v[c] = (double)s[c] * (double)wf[row * NR + c];
+            }
+        }
+    }
+    block_sum<NR>(v);
+    // the instance's blocks publish in place; the last one adds them in order
+    __shared__ bool last;
+    double *mine = part + (size_t)inst * gridDim.x * NR;
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int c = 0; c < NR; ++c) mine[(size_t)blockIdx.x * NR + c] = v[c];
+        __threadfence();
+        last = atomicAdd(cnt + inst, 1u) == (unsigned)blocks - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const int c = threadIdx.x;
+    if (c == 0) cnt[inst] = 0;
+    if (c >= NR) return;
+    double wc = 0.0;
+#pragma unroll 8
+    for (int u = 0; u < blocks; ++u) wc += __ldcg(mine + (size_t)u * NR + c);
+    BatchScal &s = sc[inst * NR + c];
+    const double rz = s.rz1 + wc;
+    if (mode == 0) {
+        if (s.done || s.pause) return;
+        s.iters += 1;
+        s.repl = 0;
+        double normb = sqrt(s.bnorm2);
+        if (normb == 0.0) normb = 1.0;
+        const double half = 0.5 * rtol * normb;
+        if (!isfinite(s.rnorm2) || !isfinite(rz)) s.done = 5;
+        else if (s.rnorm2 <= half * half || s.rnorm2 <= drop2 * s.rrep || !(rz > 0.0) || s.iters >= maxit) s.pause = 1;
+        else {
+            s.beta = rz / s.rho;
+            s.rho = rz;
+        }
+    } else if (s.done == 0 && s.repl == 2) {
+        if (!isfinite(rz) || !(rz > 0.0) || s.since >= 6) {
+            // (rtol here is a fifth of the caller's, see COARSE_MARGIN)
+            double normb = sqrt(s.bnorm2);
+            if (normb == 0.0) normb = 1.0;
+            s.done = sqrt(s.rnorm2) / normb <= rtol / COARSE_MARGIN ? 1 : 5;
+            s.repl = 0;
+        } else {
+            s.beta = mode == 2 ? 0.0 : rz / s.rho;
+            s.rho = rz;
+            s.rrep = s.rnorm2;
+            s.pause = 0;
+            s.repl = 1;
+        }
+    }
+}
+
+// p = z + W c + beta p for the running pairs (mode 0) or the restarted ones.
+template <int ND, int NR>
+__global__ void __launch_bounds__(NTHREADS) k_bcoarse_pupdate(const float *__restrict__ z,
+                                                              float *__restrict__ p, const int *__restrict__ box,
+                                                              const int *__restrict__ box_inst, const int *__restrict__ box_row,
+                                                              const int *__restrict__ inst_tab, const float *__restrict__ rel,
+                                                              const int *__restrict__ mask, int64_t nrows,
+                                                              const float *__restrict__ cvec, const BatchScal *sc, int mode)
+{
+    constexpr int NM = Modes<ND>::NM;
+    const int64_t a = (int64_t)blockIdx.x * NTHREADS + threadIdx.x;
+    if (a >= nrows) return;
+    if (mask[a] & PADDING) return;   // stays zero
+    const int b = box[a], inst = box_inst[b];
+    float x[ND], w[ND][NM];
+    load_rel<ND>(rel, nrows, a, x);
+    rigid<ND, float>(x, mask[a], w);
+    const float *q = cvec + (size_t)(inst_tab[5 * inst + 2] + box_row[b]) * NR;
+#pragma unroll
+    for (int c = 0; c < NR; ++c) {
+        const BatchScal &s = sc[inst * NR + c];
+        if (s.done || (mode ? s.repl != 1 : s.pause != 0)) continue;
+        const float beta = (float)s.beta;
+        float cc[NM];
+#pragma unroll
+        for (int m = 0; m < NM; ++m) cc[m] = __ldg(q + m * NR + c);
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+            const int64_t i = (a * ND + d) * NR + c;
+            float zz = z[i];
+#pragma unroll
+            for (int m = 0; m < NM; ++m) zz = fmaf(w[d][m], cc[m], zz);
+            p[i] = fmaf(beta, p[i], zz);
+        }
+    }
+}
+
 // p = z + W c + beta p.
 template <int ND>
 __global__ void __launch_bounds__(NTHREADS) k_coarse_pupdate(int64_t nact, const float *__restrict__ z, float *__restrict__ p,
@@ -418,10 +636,14 @@ __global__ void __launch_bounds__(NTHREADS) k_coarse_pupdate(int64_t nact, const
 
 // From COARSE_MIN_NODES active nodes on: below, the one-launch iterations without it are
 // as fast (17^3-cell tets, 5.8 k nodes: 4.9 ms with it, about 4.5 ms in one launch;
-// 40 x 11 x 9 hexes, 4.9 k nodes: 4.8 against about 9 ms).
-bool coarse_wanted(const ogb_ctx *ctx, const SellMat &S)
+// 40 x 11 x 9 hexes, 4.9 k nodes: 4.8 against about 9 ms). Solves asked for more than
+// COARSE_TIGHTEST keep block Jacobi's recurrences alone, so that their results stay the
+// ones they were to the last digits asked for: what those recurrences stop at is off the
+// solution by up to 3e-9 (quads 257 x 257 to 1e-11) or 6e-8 of single reactions (64 RVEs
+// to 1e-11), ten to fifty times more than with the coarse part, and a result moves by that.
+bool coarse_wanted(const ogb_ctx *ctx, const SellMat &S, double rtol)
 {
-    return ctx->persist && S.ninst == 1 && S.nact >= COARSE_MIN_NODES && S.xyz.p != nullptr;
+    return rtol >= COARSE_TIGHTEST && ctx->persist && S.ninst == 1 && S.nact >= COARSE_MIN_NODES && S.xyz.p != nullptr;
 }
 
 // Boxes of the active nodes (host, once per structure): equal boxes of the bounding
@@ -440,75 +662,117 @@ static int build_boxes(ogb_ctx *ctx, SellMat &S)
     std::vector<double> x((size_t)nd * nrows);
     OGB_CUDA(cudaMemcpyAsync(x.data(), S.xyz.p, x.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
     OGB_CUDA(cudaStreamSynchronize(s));
-    double lo[3], len[3], vol = 1.0;
-    int dims = 0;
-    for (int d = 0; d < nd; ++d) {
-        const auto mm = std::minmax_element(x.begin() + d * nrows, x.begin() + d * nrows + n);
-        lo[d] = *mm.first;
-        len[d] = *mm.second - *mm.first;
-        if (!(len[d] >= 0.0) || !std::isfinite(len[d])) return OGB_OK;
-        if (len[d] > 0.0) {
-            vol *= len[d];
-            ++dims;
+    const int ni = S.ninst;
+    std::vector<int> box(nrows, 0), count, first(ni + 1, 0);
+    std::vector<double> scale;   // box edge of each box's instance
+    std::vector<int> cell, id;
+    for (int q = 0; q < ni; ++q) {
+        const int64_t r0 = S.inst_row_base[q], nq = S.inst_nact[q];
+        first[q] = (int)count.size();
+        double lo[3], len[3], vol = 1.0;
+        int dims = 0;
+        for (int d = 0; d < nd && nq > 0; ++d) {
+            const auto mm = std::minmax_element(x.begin() + d * nrows + r0, x.begin() + d * nrows + r0 + nq);
+            lo[d] = *mm.first;
+            len[d] = *mm.second - *mm.first;
+            if (!(len[d] >= 0.0) || !std::isfinite(len[d])) return OGB_OK;
+            if (len[d] > 0.0) {
+                vol *= len[d];
+                ++dims;
+            }
+        }
+        if (dims == 0) {   // no active node, or one
+            count.push_back((int)nq);
+            scale.push_back(1.0);
+            for (int64_t a = r0; a < r0 + nq; ++a) box[a] = first[q];
+            continue;
+        }
+        // The smooth search directions that the coarse part brings must be resolved by the
+        // FP32 operator: the softest one, bending of the whole mesh, has about
+        // (h / L)^2 (width / L)^2 of the largest stiffness, which has to stand clear of the
+        // FP32 rounding (6e-8). 160 x 5 x 5 hexes (4e-8) do not converge with it,
+        // 290 x 58 x 58 (5e-7) do. Batches apply Ac^-1 in FP32 and keep a wider distance.
+        double longest = 0.0;
+        for (int d = 0; d < nd; ++d) longest = std::max(longest, len[d]);
+        double width = longest;
+        for (int d = 0; d < nd; ++d)
+            if (len[d] > 0.0) width = std::min(width, len[d]);
+        const double he = pow(vol / (double)nq, 1.0 / dims);
+        if (pow(he / longest, 2) * pow(width / longest, 2) < (ni > 1 ? 30.0 * COARSE_SOFTEST : COARSE_SOFTEST)) return OGB_OK;
+        const double want = ni > 1 ? std::min(64.0, std::max(4.0, nq / 128.0))
+                            : nd == 3 ? std::min(200.0, std::max(48.0, nq / 600.0))
+                                      : std::min(320.0, std::max(48.0, nq / 125.0));
+        const double h = pow(vol / want, 1.0 / dims);
+        int k[3] = {1, 1, 1};
+        for (int d = 0; d < nd; ++d) k[d] = (int)std::min(256.0, std::max(1.0, std::round(len[d] / h)));
+        const int64_t cells = (int64_t)k[0] * k[1] * k[2];
+        if (cells > 2048) return OGB_OK;
+        id.assign(cells, -1);
+        for (int64_t a = r0; a < r0 + nq; ++a) {
+            int64_t c = 0;
+            for (int d = nd - 1; d >= 0; --d) {
+                const int i = len[d] > 0.0 ? std::min(k[d] - 1, (int)((x[d * nrows + a] - lo[d]) / len[d] * k[d])) : 0;
+                c = c * k[d] + i;
+            }
+            if (id[c] < 0) {
+                id[c] = (int)count.size();
+                count.push_back(0);
+                scale.push_back(h);
+            }
+            box[a] = id[c];
+            count[id[c]]++;
         }
     }
-    if (dims == 0) return OGB_OK;
-    // The smooth search directions that the coarse part brings must be resolved by the
-    // FP32 operator: the softest one, bending of the whole mesh, has about
-    // (h / L)^2 (width / L)^2 of the largest stiffness, which has to stand clear of the
-    // FP32 rounding (6e-8). 160 x 5 x 5 hexes (4e-8) do not converge with it,
-    // 290 x 58 x 58 (5e-7) do.
-    double longest = 0.0, width = 0.0;
-    for (int d = 0; d < nd; ++d) longest = std::max(longest, len[d]);
-    width = longest;
-    for (int d = 0; d < nd; ++d)
-        if (len[d] > 0.0) width = std::min(width, len[d]);
-    const double he = pow(vol / n, 1.0 / dims);
-    if (pow(he / longest, 2) * pow(width / longest, 2) < COARSE_SOFTEST) return OGB_OK;
-    const double want = nd == 3 ? std::min(200.0, std::max(48.0, n / 600.0)) : std::min(320.0, std::max(48.0, n / 125.0)), h = pow(vol / want, 1.0 / dims);
-    int k[3] = {1, 1, 1};
-    for (int d = 0; d < nd; ++d) k[d] = (int)std::min(256.0, std::max(1.0, std::round(len[d] / h)));
-    const int64_t cells = (int64_t)k[0] * k[1] * k[2];
-    if (cells > 2048) return OGB_OK;
-    std::vector<int> cell(n), box(nrows, 0), id(cells, -1), count;
-    for (int a = 0; a < n; ++a) {
-        int q = 0;
-        for (int d = nd - 1; d >= 0; --d) {
-            const int i = len[d] > 0.0 ? std::min(k[d] - 1, (int)((x[d * nrows + a] - lo[d]) / len[d] * k[d])) : 0;
-            q = q * k[d] + i;
-        }
-        cell[a] = q;
-        if (id[q] < 0) {
-            id[q] = (int)count.size();
-            count.push_back(0);
-        }
-        box[a] = id[q];
-        count[id[q]]++;
-    }
-    const int nb = (int)count.size();
+    const int nb = (int)count.size(), nm = nd == 3 ? 6 : 3;
+    first[ni] = nb;
+    std::vector<char> on(nrows, 0);
+    for (int q = 0; q < ni; ++q)
+        for (int64_t a = S.inst_row_base[q]; a < S.inst_row_base[q] + S.inst_nact[q]; ++a) on[a] = 1;
     std::vector<double> cen((size_t)nb * nd, 0.0);
-    for (int a = 0; a < n; ++a)
-        for (int d = 0; d < nd; ++d) cen[(size_t)box[a] * nd + d] += x[d * nrows + a];
+    for (int64_t a = 0; a < nrows; ++a)
+        if (on[a])
+            for (int d = 0; d < nd; ++d) cen[(size_t)box[a] * nd + d] += x[d * nrows + a];
     std::vector<float> rel((size_t)nd * nrows, 0.f);
     for (int d = 0; d < nd; ++d)
-        for (int a = 0; a < n; ++a)
-            rel[d * nrows + a] = (float)((x[d * nrows + a] - cen[(size_t)box[a] * nd + d] / count[box[a]]) / h);
+        for (int64_t a = 0; a < nrows; ++a)
+            if (on[a]) rel[d * nrows + a] = (float)((x[d * nrows + a] - cen[(size_t)box[a] * nd + d] / count[box[a]]) / scale[box[a]]);
     // the boxes' rows, and CTAs of at most PART_ROWS of them
-    constexpr int PART_ROWS = 1536;
-    std::vector<int> start(nb + 1, 0), list(n), part, bp(nb + 1, 0);
+    const int PART_ROWS = ni > 1 ? 512 : 1536;   // a warp's, a CTA's
+    std::vector<int> start(nb + 1, 0), list(n > 0 ? n : 1), part, bp(nb + 1, 0), box_inst(nb), box_row(nb), inst(5 * ni);
+    std::vector<int64_t> mat(ni + 1, 0);
     for (int i = 0; i < nb; ++i) start[i + 1] = start[i] + count[i];
     std::vector<int> fill(start.begin(), start.end() - 1);
-    for (int a = 0; a < n; ++a) list[fill[box[a]]++] = a;
+    for (int64_t a = 0; a < nrows; ++a)
+        if (on[a]) list[fill[box[a]]++] = (int)a;
+    C.nparts = 0;
     for (int i = 0; i < nb; ++i) {
         bp[i] = (int)part.size();
         for (int q = start[i]; q < start[i + 1]; q += PART_ROWS) part.push_back(q);
     }
     bp[nb] = (int)part.size();
     C.nparts = (int)part.size();
+    if (C.nparts == 0) return OGB_OK;
     part.push_back(n);
-    C.nm = nd == 3 ? 6 : 3;
-    C.nc = nb * C.nm;
-    C.ncp = (int)ceil_div(C.nc, GJ) * GJ;
+    C.ninst = ni;
+    C.nm = nm;
+    C.nvec = C.maxblocks = 0;
+    for (int q = 0; q < ni; ++q) {
+        const int nc = (first[q + 1] - first[q]) * nm, ncp = (int)ceil_div(nc, GJ) * GJ;
+        for (int i = first[q]; i < first[q + 1]; ++i) {
+            box_inst[i] = q;
+            box_row[i] = (i - first[q]) * nm;
+        }
+        inst[5 * q] = nc;
+        inst[5 * q + 1] = ncp;
+        inst[5 * q + 2] = C.nvec;
+        inst[5 * q + 3] = first[q];
+        inst[5 * q + 4] = first[q + 1] - first[q];
+        mat[q + 1] = mat[q] + (int64_t)ncp * ncp;
+        C.nvec += ncp;
+        C.maxblocks = std::max(C.maxblocks, ncp / GJ);
+    }
+    C.nc = inst[0];
+    C.ncp = inst[1];
     auto up = [&](auto &dst, const auto &src) -> int {
         OGB_CHECK(dst.alloc(src.size()));
         OGB_CUDA(cudaMemcpyAsync(dst.p, src.data(), src.size() * sizeof(src[0]), cudaMemcpyHostToDevice, s));
@@ -519,24 +783,30 @@ static int build_boxes(ogb_ctx *ctx, SellMat &S)
     OGB_CHECK(up(C.list, list));
     OGB_CHECK(up(C.part, part));
     OGB_CHECK(up(C.box_part, bp));
+    OGB_CHECK(up(C.box_inst, box_inst));
+    OGB_CHECK(up(C.box_row, box_row));
+    OGB_CHECK(up(C.inst, inst));
+    OGB_CHECK(up(C.inst_mat, mat));
     OGB_CUDA(cudaStreamSynchronize(s));
-    OGB_CHECK(C.fixed.alloc((size_t)C.nc * C.nc));
+    C.nfix = (size_t)mat[ni];
+    OGB_CHECK(C.fixed.alloc(C.nfix));
     OGB_CHECK(C.maxd.alloc(1));
-    OGB_CHECK(C.a.alloc((size_t)C.ncp * C.ncp));
-    OGB_CHECK(C.b.alloc((size_t)C.ncp * C.ncp));
-    OGB_CHECK(C.d.alloc(GJ * GJ));
-    OGB_CHECK(C.parts.alloc((size_t)C.nparts * C.nm));
-    OGB_CHECK(C.c.alloc(C.ncp));
+    OGB_CHECK(C.a.alloc(C.nfix));
+    OGB_CHECK(C.b.alloc(C.nfix));
+    OGB_CHECK(C.d.alloc((size_t)ni * GJ * GJ));
+    OGB_CHECK(C.parts.alloc((size_t)C.nparts * nm * 4));   // four load cases at most (floats: half of it)
+    OGB_CHECK(C.c.alloc((size_t)C.nvec * 4));
+    OGB_CHECK(C.inv32.alloc(C.nfix));
     // the rows that add to Ac
     {
         DBuf<int64_t> flag;
         OGB_CHECK(flag.alloc(n + 1));
         OGB_CHECK(C.need.alloc(n));
-        k_coarse_need<<<(unsigned)ceil_div(n + 1, 256), 256, 0, s>>>(n, S.sl_ptr.p, S.sl_width.p, S.col.p, C.box.p, S.free_mask.p,
+        k_coarse_need<<<(unsigned)ceil_div(n + 1, 256), 256, 0, s>>>(n, C.list.p, S.sl_ptr.p, S.sl_width.p, S.col.p, C.box.p, S.free_mask.p,
                                                                     (1 << nd) - 1, flag.p);
         int64_t total = 0;
         OGB_CHECK(exclusive_scan_i64(ctx, flag.p, flag.p, n + 1, &total));
-        k_coarse_list<<<(unsigned)ceil_div(n, 256), 256, 0, s>>>(n, flag.p, C.need.p);
+        k_coarse_list<<<(unsigned)ceil_div(n, 256), 256, 0, s>>>(n, C.list.p, flag.p, C.need.p);
         count_launch(ctx, 2);
         OGB_CUDA(cudaGetLastError());
         OGB_CUDA(cudaStreamSynchronize(s));   // flag is freed
@@ -555,30 +825,31 @@ int refresh_coarse(ogb_ctx *ctx, SellMat &S, int64_t version)
     if (!C.ok || C.version == version) return OGB_OK;
     cudaStream_t s = ctx->stream;
     const int64_t nrows = (int64_t)S.nslices * 32;
-    OGB_CUDA(cudaMemsetAsync(C.fixed.p, 0, (size_t)C.nc * C.nc * sizeof(long long), s));
+    OGB_CUDA(cudaMemsetAsync(C.fixed.p, 0, C.nfix * sizeof(long long), s));
     OGB_CUDA(cudaMemsetAsync(C.maxd.p, 0, sizeof(unsigned long long), s));
     const unsigned g = (unsigned)ceil_div(C.nlist > 0 ? C.nlist : 1, 128);
     unsigned long long *F = reinterpret_cast<unsigned long long *>(C.fixed.p);
     if (S.nd == 3) {
-        k_max_diag<3><<<num_sms() * 2, 256, 0, s>>>(S.nact, S.diag.p, S.v64.p, C.maxd.p);
+        k_max_diag<3><<<num_sms() * 2, 256, 0, s>>>((int)nrows, S.diag.p, S.v64.p, C.maxd.p);
         k_coarse_matrix<3><<<g, 128, 0, s>>>(C.nlist, C.need.p, S.sl_ptr.p, S.sl_width.p, S.col.p, S.v64.p, C.box.p, C.rel.p, S.free_mask.p,
-                                             nrows, C.nc, C.maxd.p, F);
+                                             nrows, C.box_inst.p, C.box_row.p, C.inst.p, C.inst_mat.p, C.maxd.p, F);
     } else {
-        k_max_diag<2><<<num_sms() * 2, 256, 0, s>>>(S.nact, S.diag.p, S.v64.p, C.maxd.p);
+        k_max_diag<2><<<num_sms() * 2, 256, 0, s>>>((int)nrows, S.diag.p, S.v64.p, C.maxd.p);
         k_coarse_matrix<2><<<g, 128, 0, s>>>(C.nlist, C.need.p, S.sl_ptr.p, S.sl_width.p, S.col.p, S.v64.p, C.box.p, C.rel.p, S.free_mask.p,
-                                             nrows, C.nc, C.maxd.p, F);
+                                             nrows, C.box_inst.p, C.box_row.p, C.inst.p, C.inst_mat.p, C.maxd.p, F);
     }
-    const int64_t nn = (int64_t)C.ncp * C.ncp;
-    k_coarse_convert<<<(unsigned)ceil_div(nn, 256), 256, 0, s>>>(C.nc, C.ncp, C.fixed.p, C.maxd.p, C.a.p);
-    double *A = C.a.p, *B = C.b.p;
-    const int nb = C.ncp / GJ;
-    for (int k = 0; k < nb; ++k) {
-        k_gj_diag<<<1, NTHREADS, 0, s>>>(C.ncp, k, A, C.d.p);
-        k_gj_update<<<dim3(nb, nb), NTHREADS, 0, s>>>(C.ncp, k, A, C.d.p, B);
-        std::swap(A, B);
+    k_coarse_convert<<<dim3((unsigned)std::min<int64_t>(ceil_div((int64_t)C.maxblocks * GJ * C.maxblocks * GJ, 256), 4096), C.ninst), 256, 0, s>>>(
+        C.inst.p, C.inst_mat.p, C.fixed.p, C.maxd.p, C.a.p);
+    // (a smaller matrix is done after its own number of steps: its inverse is in the
+    // buffer of that step's parity)
+    for (int k = 0; k < C.maxblocks; ++k) {
+        const double *A = k & 1 ? C.b.p : C.a.p;
+        k_gj_diag<<<C.ninst, NTHREADS, 0, s>>>(C.inst.p, C.inst_mat.p, k, A, C.d.p);
+        k_gj_update<<<dim3(C.maxblocks, C.maxblocks, C.ninst), NTHREADS, 0, s>>>(C.inst.p, C.inst_mat.p, k, A, C.d.p, k & 1 ? C.a.p : C.b.p);
     }
-    C.inv = A;
-    count_launch(ctx, 3 + 2 * nb);
+    C.inv = C.ncp / GJ & 1 ? C.b.p : C.a.p;
+    k_coarse_inv32<<<dim3(256, C.ninst), 256, 0, s>>>(C.inst.p, C.inst_mat.p, C.a.p, C.b.p, C.inv32.p);
+    count_launch(ctx, 3 + 2 * C.maxblocks);
     OGB_CUDA(cudaGetLastError());
     C.version = version;
     return OGB_OK;
@@ -601,6 +872,48 @@ int launch_coarse(ogb_ctx *ctx, SellMat &S, const float *r, const float *z, floa
     else k_coarse_pupdate<2><<<gp, NTHREADS, 0, s>>>(S.nact, z, p, C.box.p, C.rel.p, S.free_mask.p, nrows, C.c.p, sc);
     count_launch(ctx, 3);
     return OGB_OK;
+}
+
+// Batches that the one-launch form does not take: from about a thousand nodes per
+// instance on.
+bool batch_coarse_wanted(const ogb_ctx *ctx, const SellMat &S, double rtol)
+{
+    return rtol >= COARSE_TIGHTEST && ctx->persist && ctx->mixed_diff && ctx->mixed_bj && S.xyz.p != nullptr && S.nact >= (int64_t)1024 * S.ninst;
+}
+
+template <int ND, int NR>
+static int batch_coarse_nr(ogb_ctx *ctx, SellMat &S, const float *r, const float *z, float *p, double *part, unsigned int *cnt,
+                           BatchScal *sc, double rtol, double drop2, int maxit, int mode)
+{
+    Coarse &C = S.coarse;
+    cudaStream_t s = ctx->stream;
+    const int64_t nrows = (int64_t)S.nslices * 32;
+    const unsigned gx = (unsigned)ceil_div((int64_t)C.maxblocks * GJ, NTHREADS / 32);
+    float *parts = reinterpret_cast<float *>(C.parts.p), *c = reinterpret_cast<float *>(C.c.p);
+    k_bcoarse_restrict<ND, NR><<<(unsigned)ceil_div(C.nparts, NTHREADS / 32), NTHREADS, 0, s>>>(
+        C.nparts, C.part.p, C.list.p, C.box.p, C.box_inst.p, C.rel.p, S.free_mask.p, nrows, r, parts, sc, mode);
+    k_bcoarse_solve<NR><<<dim3(gx, C.ninst), NTHREADS, (size_t)C.maxblocks * GJ * NR * sizeof(float), s>>>(
+        C.inst.p, C.inst_mat.p, C.nm, C.box_part.p, parts, C.inv32.p, c, part, cnt, sc, rtol, drop2, maxit, mode);
+    k_bcoarse_pupdate<ND, NR><<<(unsigned)ceil_div(nrows, NTHREADS), NTHREADS, 0, s>>>(
+        z, p, C.box.p, C.box_inst.p, C.box_row.p, C.inst.p, C.rel.p, S.free_mask.p, nrows, c, sc, mode);
+    return OGB_OK;
+}
+
+int launch_batch_coarse(ogb_ctx *ctx, SellMat &S, int nr, const float *r, const float *z, float *p, double *part,
+                        unsigned int *cnt, BatchScal *sc, double rtol, double drop2, int maxit, int mode)
+{
+#define OGB_BC(ND_, NR_) \
+    if (S.nd == ND_ && nr == NR_) return batch_coarse_nr<ND_, NR_>(ctx, S, r, z, p, part, cnt, sc, rtol, drop2, maxit, mode)
+    OGB_BC(2, 1);
+    OGB_BC(2, 2);
+    OGB_BC(2, 3);
+    OGB_BC(2, 4);
+    OGB_BC(3, 1);
+    OGB_BC(3, 2);
+    OGB_BC(3, 3);
+    OGB_BC(3, 4);
+#undef OGB_BC
+    return fail(OGB_E_STATE, "batched coarse preconditioner: no kernel of this shape");
 }
 
 }  // namespace ogb

@@ -85,8 +85,7 @@ __device__ void quad_grad_at(const R (&x)[4][2], R ksi, R eta, R (&g)[4][2], R &
         j10 += dn1[i] * x[i][0]; j11 += dn1[i] * x[i][1];
     }
     det = j00 * j11 - j01 * j10;
-    const R rd = R(1) / det;
-    const R i00 = j11 * rd, i01 = -j01 * rd, i10 = -j10 * rd, i11 = j00 * rd;
+    const R i00 = j11 / det, i01 = -j01 / det, i10 = -j10 / det, i11 = j00 / det;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         g[i][0] = i00 * dn0[i] + i01 * dn1[i];

@@ -125,13 +125,14 @@ struct PcgScal {
 struct BatchScal {
     double bnorm2, rho, pq, rnorm2, alpha, beta;
     double mark;   // mixed precision: FP64 residual^2 at the last halving
+    double rz1;    // coarse part still to come: r.z of the block Jacobi part
     double rrep;   // mixed precision: FP64 residual^2 at the last replacement (the drop test's reference)
     int done;      // 0 running, 1 converged, 2 breakdown, 3 zero pivot, 4 iteration limit, 5 stalled (mixed),
                    // 6 a wait of the one-launch form timed out
     int iters;
     int pause;     // mixed precision: waits for the next FP64 residual replacement
     int since;     // mixed precision: replacements since the FP64 residual last halved
-    int repl;      // mixed precision: replaced in the last replacement pass, p update pending
+    int repl;      // mixed precision: 1 replaced in the last pass, p update pending; 2 its r.z pending too (coarse part)
     int pad_;
 };
 
@@ -178,10 +179,16 @@ struct Coarse {
     DBuf<int> need;                            // rows that add to the coarse matrix
     int nlist = 0;
     DBuf<float> rel;                           // position in the box, planes
+    DBuf<int> box_inst, box_row;               // instance of a box; its first row in the instance's coarse matrix
+    DBuf<int> inst;                            // per instance: equations, padded, first row in c, first box, boxes
+    DBuf<int64_t> inst_mat;                    // per instance: its matrix in fixed, a, b
+    size_t nfix = 0;
+    int ninst = 0, maxblocks = 0, nvec = 0;    // instances; blocks of the largest matrix; rows of c
     DBuf<long long> fixed;
     DBuf<unsigned long long> maxd;
     DBuf<double> a, b, d, parts, c;
-    const double *inv = nullptr;
+    DBuf<float> inv32;                         // FP32 copy of all inverses (batches)
+    const double *inv = nullptr;               // of the first instance
     int64_t version = -1;
 };
 
@@ -483,8 +490,18 @@ int batch_persist_run(ogb_mtrx *m, const BatchPersistPlan &P, int nr, bool mixed
 
 // coarse.cu: coarse part of the mixed preconditioner.
 constexpr int COARSE_MIN_NODES = 4096;
-bool coarse_wanted(const ogb_ctx *ctx, const SellMat &S);
+// Solves with the coarse part go on to this share of the tolerance: they reach it in a
+// few more iterations, and what they stop at is then no further from the solution than
+// what the longer recurrences without it end with.
+constexpr double COARSE_MARGIN = 0.2;
+constexpr double COARSE_TIGHTEST = 1e-10;   // tolerances below it: see coarse_wanted
+bool coarse_wanted(const ogb_ctx *ctx, const SellMat &S, double rtol);
 int refresh_coarse(ogb_ctx *ctx, SellMat &S, int64_t version);
+// ... of a batch: c for every right-hand side and the pairs' scalars (mode 0: an iteration, 1: a replacement
+// pass, 2: the first one), then p.
+bool batch_coarse_wanted(const ogb_ctx *ctx, const SellMat &S, double rtol);
+int launch_batch_coarse(ogb_ctx *ctx, SellMat &S, int nr, const float *r, const float *z, float *p, double *part,
+                        unsigned int *cnt, BatchScal *sc, double rtol, double drop2, int maxit, int mode);
 int launch_coarse(ogb_ctx *ctx, SellMat &S, const float *r, const float *z, float *p, double *part, unsigned int *count,
                   PcgScal *sc, int maxit, int replace, int first);
 

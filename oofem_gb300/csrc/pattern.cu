@@ -668,15 +668,15 @@ __global__ void k_ns_of_eq(int nnodes, int ndofpn, const int *eq, const int *act
     }
 }
 
-// Coordinates (planes) and free DOFs of every node row; padding rows: zero, all free
-// (an identity block that no other row refers to).
+// Coordinates (planes) and free DOFs of every node row; padding rows (identity blocks
+// that no other row refers to): zero and 8.
 __global__ void k_row_geometry(int nrows, int nd, const int *__restrict__ rownode, const double *__restrict__ coords,
                                const int *__restrict__ eq, double *__restrict__ xyz, int *__restrict__ mask)
 {
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= nrows) return;
     const int A = rownode[a];
-    int f = A < 0 ? (1 << nd) - 1 : 0;
+    int f = A < 0 ? 8 : 0;
     for (int d = 0; d < nd; ++d) {
         xyz[(size_t)d * nrows + a] = A < 0 ? 0.0 : coords[(size_t)A * nd + d];
         if (A >= 0 && eq[(size_t)A * nd + d] > 0) f |= 1 << d;

@@ -47,6 +47,32 @@ __device__ __forceinline__ void block_sum(double (&v)[NV])
         for (int k = 0; k < NV; ++k) v[k] = res[k];
 }
 
+// The sum in the order of the warps' shuffles, then the warps in index order, for the
+// residual replacements of batches: a few dozen launches of a solve, whose results
+// then do not depend on which of the two sums the library uses.
+template <int NV>
+__device__ __forceinline__ void block_sum_shuffle(double (&v)[NV])
+{
+    __shared__ double red[NV][NTHREADS / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const double s = warp_sum(v[k]);
+        if (lane == 0) red[k][warp] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            double s = 0;
+#pragma unroll
+            for (int w = 0; w < NTHREADS / 32; ++w) s += red[k][w];
+            v[k] = s;
+        }
+    }
+    __syncthreads();
+}
+
 // Block reduction of per-thread values of type T: the warp sum stays in T (an
 // FP32 warp sum costs no FP64 instruction), the warps are added in FP64 in
 // index order, one value per lane (in one thread value after value the additions

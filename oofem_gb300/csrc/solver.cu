@@ -1888,7 +1888,7 @@ int pcg_ic_core(ogb_mtrx *m, const Op &op, const double *b, double *x, double rt
 // FP32 and the SpMV multiplies and accumulates in FP32.
 template <class X, class P>
 int pcg_mixed_core(ogb_mtrx *m, const Op &op, const double *v64, const float *v32, const double *b, double *x,
-                   double rtol, int maxit, ogb_solve_info *info, bool *stalled)
+                   const double rtol_asked, int maxit, ogb_solve_info *info, bool *stalled)
 {
     ogb_ctx *ctx = m->ctx;
     cudaStream_t s = ctx->stream;
@@ -1899,12 +1899,13 @@ int pcg_mixed_core(ogb_mtrx *m, const Op &op, const double *v64, const float *v3
     // (the fused form is a cooperative launch: at most its occupancy per SM)
     // (with the coarse part of the preconditioner z is not complete after the update)
     bool coarse = sizeof(X) == 4 && sizeof(P) == 4 && op.sell && ctx->mixed_bj && m->precond == 1 && ctx->mixed_diff &&
-                  ctx->mixed_x64 && !ctx->mixed_sum32 && !ctx->mixed_orth && m->coarse_off != m->version && coarse_wanted(ctx, *op.S);
+                  ctx->mixed_x64 && !ctx->mixed_sum32 && !ctx->mixed_orth && m->coarse_off != m->version && coarse_wanted(ctx, *op.S, rtol_asked);
     if (coarse) {
         OGB_CHECK(refresh_coarse(ctx, const_cast<SellMat &>(*op.S), m->version));
         coarse = op.S->coarse.ok;
     }
     m->last_coarse = coarse;
+    const double rtol = coarse ? COARSE_MARGIN * rtol_asked : rtol_asked;
     const bool fuse = ctx->fused_update && op.sell && !coarse;
     const void *ufn = op.sell ? bj_update_fn(op.S->nd, ctx->mixed_x64 ? (ctx->mixed_sum32 ? 2 : 1) : (ctx->mixed_sum32 ? 0 : 3), fuse)
                               : nullptr;
@@ -2089,13 +2090,17 @@ int pcg_mixed_core(ogb_mtrx *m, const Op &op, const double *v64, const float *v3
         achieved = sqrt(h2[0]) / normb;
         if (achieved <= rtol) { status = OGB_OK; break; }
         if (!isfinite(achieved)) { status = OGB_E_BREAKDOWN; break; }
-        if (iters >= maxit) break;
+        if (iters >= maxit) {
+            if (achieved <= rtol_asked) status = OGB_OK;
+            break;
+        }
         // stagnation: the FP32 operator no longer brings the FP64 residual down
         // (six replacement cycles without halving it, or a breakdown of the
         // FP32 recurrences); the caller finishes the solve in FP64
         if (!(achieved < 0.5 * mark)) {
             if (++since_mark >= (coarse ? 2 : 6) || replacements > 400) {
-                *stalled = true;
+                if (achieved <= rtol_asked) status = OGB_OK;
+                else *stalled = true;
                 break;
             }
         } else {

@@ -390,3 +390,39 @@ def test_batch_in_one_launch(kind, sides, nrhs, native_lib):
         for k in range(nrhs):
             assert rel(a[0][k], f[0][k]) < tol and rel(a[1][k], f[1][k]) < tol, (rel(a[0][k], f[0][k]), rel(a[1][k], f[1][k]))
         assert a[3] < f[3]
+
+
+@pytest.mark.parametrize("kind,sides,nrhs", [("rve", (100, 128, 31, 110), 3), ("rve", (230, 190, 2, 1, 40), 1),
+                                             ("rve", (140, 133), 4), ("tet", (33, 40, 10), 1), ("tet", (20, 24, 26), 2)])
+def test_batch_coarse_preconditioner(kind, sides, nrhs, native_lib):
+    """Larger mixed batches with the coarse part of the preconditioner (instances of
+    very different sizes, one without a free DOF, one with a single node) against
+    block or scalar Jacobi alone (kept by contexts that choose a form of the
+    launches): every pair meets the tolerance on its FP64 residual, solutions agree
+    to it times the condition number (1e-10, below 1e5), fewer iterations, bitwise
+    reproducible."""
+    from oofem_gb300 import meshgen as mg
+    if kind == "rve":
+        meshes = [mg.quad_rve(n, seed=i) for i, n in enumerate(sides)]
+        bc = np.stack([np.concatenate([mg.rve_bc_values(m, c % 3) * (1 + c // 3) for m in meshes]) for c in range(nrhs)])
+    else:
+        meshes = [mg.tet_cube_linear(n, jitter=0.15, seed=i) for i, n in enumerate(sides)]
+        bc = np.stack([np.concatenate([m.bc_value for m in meshes]) * (1 + c) for c in range(nrhs)])
+    big, starts = mg.concat_meshes(meshes)
+    out = []
+    for forced in (False, False, True):
+        c = native_lib.Context(0)
+        if forced:
+            c.set_option(native_lib.OPT_BATCH_X64, 0)
+        model = native_lib.GpuModel(c, big)
+        model.set_instances(starts)
+        A = native_lib.GpuCsrMtrx(c)
+        u, reac, its, ach, st = model.batch_linear_static(A, bc, rtol=1e-10, precision=native_lib.PREC_MIXED)
+        assert (st == 0).all() and (ach <= 1e-10).all(), (st, ach)
+        out.append((u, reac, its))
+    a, b, f = out
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[2], b[2])
+    for k in range(nrhs):
+        assert rel(a[0][k], f[0][k]) < 1e-5 and rel(a[1][k], f[1][k]) < 1e-5
+    print(kind, sides, "mean iterations", a[2].mean(), "without", f[2].mean())
+    assert a[2].sum() < f[2].sum()
