@@ -79,7 +79,14 @@ OGB_API void *ogb_ctx_stream(ogb_ctx *ctx);                 /* cudaStream_t */
 OGB_API int ogb_ctx_synchronize(ogb_ctx *ctx);
 /* Number of kernels this library launched on the context since creation. */
 OGB_API int64_t ogb_ctx_kernel_launches(ogb_ctx *ctx);
-/* Tuning options of a context (no reference counterpart):
+/* Tuning options of a context (no reference counterpart). By themselves, small and
+ * middle-sized solves run their CG iterations in one launch, and larger mixed ones
+ * add a coarse part (rigid motions of boxes of nodes) to the block-Jacobi
+ * preconditioner. An option set to a value that chooses a form of the per-iteration
+ * launches (any value of OGB_OPT_MIXED_X64, _FUSED_UPDATE, _BATCH_FORM, _BATCH_X64; a
+ * value other than the default of OGB_OPT_MIXED_VEC32, _DIFF, _P32, _BLOCK_JACOBI,
+ * OGB_OPT_SPMV_VARIANT, _SPMV_HALF, _HALF_FORM, _UPDATE_BLOCKS) makes the context keep
+ * to those launches, with block or scalar Jacobi alone.
  *   OGB_OPT_MIXED_VEC32 (0/1): mixed solves keep the CG vectors in FP32 instead
  *   of FP64 (default 1). */
 #define OGB_OPT_MIXED_VEC32 1
@@ -213,9 +220,9 @@ OGB_API int ogb_mtrx_set_at(ogb_mtrx *m, int i, int j, double value);
  * src/core/iml/iluprecond.C), 4 = incomplete Cholesky
  * (CompCol_ICPreconditioner, src/core/iml/icprecond.C). For 2 and 4 the
  * reference's factorization loop runs on the host once per matrix version and
- * the two triangular solves run level by level on the device (FP64 only,
- * equation-space CSR operator). 3 (threshold ILU of a DynCompRow matrix) gives
- * OGB_E_ARG. Batched solves (ogb_batch_*) use the diagonal preconditioner only. */
+ * the two triangular solves run on the device as a dataflow over the rows (FP64
+ * only, equation-space CSR operator). 3 (threshold ILU of a DynCompRow matrix) gives
+ * OGB_E_ARG. Batched solves (ogb_batch_*) do not use 2 and 4. */
 OGB_API int ogb_mtrx_set_preconditioner(ogb_mtrx *m, int type);
 /* Node-block SpMV forms in use for this matrix (0 = not tuned yet, or no
  * node-block copy): the OGB_OPT_SPMV_VARIANT numbers 1..4 chosen for FP64 and
@@ -284,11 +291,14 @@ OGB_API int ogb_pcg_solve_noalloc(int n, const int64_t *rowptr_dev, const int *c
 #define OGB_LS_GPUPCG 9
 OGB_API int ogb_mtrx_set_solver(ogb_mtrx *m, int lstype);
 /* SparseMtrx::factorized (skyline.C:429-491): factor the current values (the
- * factor is kept until the next mutation). The factor is a dense band of
- * neq x (bw+1) doubles, bw the half bandwidth of the pattern (OGB_E_LIMIT when
- * it does not fit in device memory); OGB_E_ZERODIAG names a zero pivot. */
+ * factor is kept until the next mutation). The equations are reordered for a small
+ * half bandwidth bw (kept with the structure) and the band is factored from both
+ * ends; the factor is (neq + about bw) x (bw+1) doubles (OGB_E_LIMIT when it does
+ * not fit in device memory). A matrix that meets a zero pivot this way is factored
+ * in its own order, from one end; OGB_E_ZERODIAG names a zero pivot met there. */
 OGB_API int ogb_ldlt_factorize(ogb_mtrx *m);
-/* Half bandwidth of the current factor (OGB_E_STATE before ogb_ldlt_factorize). */
+/* Half bandwidth of the pattern in the equations' own order (OGB_E_STATE before
+ * ogb_ldlt_factorize). */
 OGB_API int ogb_ldlt_bandwidth(ogb_mtrx *m, int *bandwidth);
 /* LDLTFactorization::solve (ldltfact.C:50-63): x = A^-1 b, factoring first when
  * the values changed. Host vectors of neq doubles / device vectors (_dev). */

@@ -365,12 +365,15 @@ int64_t ogb_ctx_kernel_launches(ogb_ctx *ctx) { return ctx ? ctx->launches : 0; 
 int ogb_ctx_set_option(ogb_ctx *ctx, int option, int64_t value)
 {
     if (!ctx) return fail(OGB_E_ARG, "null context");
-    switch (option) {   // options that choose a form of the per-iteration launches keep to those launches
-    case OGB_OPT_MIXED_VEC32: case OGB_OPT_MIXED_DIFF: case OGB_OPT_MIXED_P32: case OGB_OPT_MIXED_X64:
-    case OGB_OPT_SPMV_VARIANT: case OGB_OPT_SPMV_HALF: case OGB_OPT_MIXED_BLOCK_JACOBI: case OGB_OPT_UPDATE_BLOCKS:
-    case OGB_OPT_HALF_FORM: case OGB_OPT_FUSED_UPDATE: case OGB_OPT_BATCH_FORM: case OGB_OPT_BATCH_X64:
-        ctx->persist = false;
+    // a value that chooses a form of the per-iteration launches keeps to those launches
+    switch (option) {
+    case OGB_OPT_MIXED_VEC32: case OGB_OPT_MIXED_DIFF: case OGB_OPT_MIXED_BLOCK_JACOBI: case OGB_OPT_SPMV_HALF:
+        if (value != 1) ctx->persist = false;
         break;
+    case OGB_OPT_MIXED_P32: case OGB_OPT_SPMV_VARIANT: case OGB_OPT_UPDATE_BLOCKS: case OGB_OPT_HALF_FORM:
+        if (value != 0) ctx->persist = false;
+        break;
+    case OGB_OPT_MIXED_X64: case OGB_OPT_FUSED_UPDATE: case OGB_OPT_BATCH_FORM: case OGB_OPT_BATCH_X64: ctx->persist = false; break;
     default: break;
     }
     switch (option) {
