@@ -94,64 +94,92 @@ __global__ void k_ldl_fill(int n, int mid, const int64_t *__restrict__ rowptr, c
 
 // Diagonal block of panel [k0, k0 + P) of a band (P <= 32): L D L^T and the inverse X
 // of its unit triangle together, as row operations on the full symmetric 32 x 32
-// block E (a warp holds rows warp + 8 q, a lane one column). In step j row j's owner
-// publishes W = E(j, :) / d_j (with 1 / d_j in column j), and every row r > j
-// subtracts E(r, j) W. Right of the diagonal that is the elimination of A, left of
-// it and in column j the same operations build X = L^-1. One barrier per step; the
-// chain is the pivot's reciprocal, which the next row's owner takes right after
-// that row's update, its first of the step: 0.75 us per step, most of it FP64
-// latency. (Three barriers and a division in every row: 52 us per block; this
-// scheme 24.8 us in eight warps and 24.2 us in 32, so the CTA that has updated the
-// block can go on with it.) A zero or
-// non-finite pivot sets *status to the 1-based equation of the band (negative:
-// second band) and stops every later launch.
-constexpr int ROWS_PER_WARP = PANEL / (NTHREADS / 32);
-__device__ __forceinline__ void factor_block(const Bands &B, int band, int k0, int P, double (&e)[ROWS_PER_WARP],
-                                             double (&W)[2][PANEL], int &bad, int *status)
+// block E in shared memory (lane = column). In step j every row r > j subtracts
+// E(r, j) W, W = E(j, :) / d_j with 1 / d_j in column j: right of the diagonal that is
+// the elimination of A, left of it and in column j the same operations build
+// X = L^-1. The chain of a step is the next row's update, its pivot's reciprocal and
+// its scaling. A warp issues one FP64 instruction per 64 cycles, two warps on one of
+// the SM's four partitions half as many each, so this chain has a partition to itself:
+// warp PIVOT takes the next row (handed over by its owner one step earlier), the other
+// rows are held by the six warps of the other three partitions. One barrier per step.
+// (Three barriers and a division in every row: 52 us per block; rows in eight warps,
+// the reciprocal taken by the next row's owner among its other updates: 24.8 us; this:
+// 22.4 us. A dependent FP64 division takes 364 cycles, 688 beside a second warp.) A zero
+// or non-finite pivot sets *status to the 1-based equation of the band (negative: second
+// band) and stops every later launch.
+constexpr int PIVOT = 3, ROW_WARPS = 6, ROWS_PER_WARP = (PANEL + ROW_WARPS - 1) / ROW_WARPS;
+struct BlockShared {
+    double E[PANEL][PANEL + 1], W[2][PANEL], R[2][PANEL], sub[PANEL];   // R: the row handed over; sub: L(r, r - 1)
+    int bad;
+};
+
+__device__ __forceinline__ void factor_block(const Bands &B, int band, int k0, int P, BlockShared &S, int *status)
 {
     const int bw = B.bw, warp = threadIdx.x >> 5, c = threadIdx.x & 31;
+    const int wi = warp < 3 ? warp : warp > 3 && warp < 7 ? warp - 1 : -1;   // warps 3 and 7 share a partition
     double *A = B.a[band];
     const int64_t ld = (int64_t)bw + 1;
-    double l[ROWS_PER_WARP];
+    double e[ROWS_PER_WARP], l[ROWS_PER_WARP];
+    __syncthreads();   // E is complete
 #pragma unroll
-    for (int q = 0; q < ROWS_PER_WARP; ++q) l[q] = 0.0;
-    if (threadIdx.x == 0) bad = 0;
+    for (int q = 0; q < ROWS_PER_WARP; ++q) {
+        const int r = wi + ROW_WARPS * q;
+        e[q] = wi >= 0 && r < PANEL ? S.E[r][c] : 0.0;
+        l[q] = 0.0;
+    }
+    if (warp == 0) S.R[1][c] = S.E[1][c];
+    if (threadIdx.x == 0) S.bad = 0;
     __syncthreads();
-    auto publish = [&](int j, double row) {   // row j's warp
+    auto pivot = [&](int j, double row) {   // row j is final: its scaled copy
         const double d = __shfl_sync(0xffffffffu, row, j);
-        if ((!(d != 0.0) || !isfinite(d)) && c == 0) bad = j + 1;
-        const double r = 1.0 / d;
-        W[j & 1][c] = c == j ? r : row * r;
+        const double q = 1.0 / d, w = c == j ? q : row * q;
+        S.W[j & 1][c] = w;
+        S.E[j][c] = row;
+        // by the bits: an FP64 comparison would wait its turn in the chain
+        const unsigned hi = (unsigned)__double2hiint(d) & 0x7fffffffu;
+        if ((hi >= 0x7ff00000u || !(hi | (unsigned)__double2loint(d))) && c == 0) S.bad = j + 1;
+        return w;
     };
-    if (warp == 0) publish(0, e[0]);
-#pragma unroll
-    for (int jq = 0; jq < ROWS_PER_WARP; ++jq)
+    double own = 0.0;   // PIVOT's copy of the current W
+    if (warp == PIVOT) own = pivot(0, S.E[0][c]);
 #pragma unroll 1
-        for (int jw = 0; jw < NTHREADS / 32; ++jw) {
-            const int j = jw + (NTHREADS / 32) * jq;
-            if (j >= P) break;
-            __syncthreads();
-            if (bad) {
-                if (threadIdx.x == 0) atomicCAS(status, 0, band ? -(k0 + bad) : k0 + bad);
-                return;   // every thread read the same flag after the barrier: a uniform exit
+    for (int j = 0; j < P; ++j) {
+        __syncthreads();
+        if (S.bad == j + 1) {   // set before the barrier; a later row's is left for its own step
+            if (threadIdx.x == 0) atomicCAS(status, 0, band ? -(k0 + j + 1) : k0 + j + 1);
+            return;   // uniform over the CTA
+        }
+        if (warp == PIVOT) {
+            if (j + 1 < P) {
+                const double row = S.R[(j + 1) & 1][c];
+                const double f = __shfl_sync(0xffffffffu, row, j);
+                const double t = fma(-f, own, c == j ? 0.0 : row);
+                if (c == j) S.sub[j + 1] = -t;
+                own = pivot(j + 1, t);
             }
-            const double w = W[j & 1][c];
+        } else if (wi >= 0) {
+            const double w = S.W[j & 1][c];
 #pragma unroll
-            for (int q = jq; q < ROWS_PER_WARP; ++q) {
-                const int r = warp + (NTHREADS / 32) * q;
-                if (r <= j) continue;
+            for (int q = 0; q < ROWS_PER_WARP; ++q) {
+                const int r = wi + ROW_WARPS * q;
+                if (r <= j + 1 || r >= P) continue;
                 const double f = __shfl_sync(0xffffffffu, e[q], j);
                 const double t = fma(-f, w, c == j ? 0.0 : e[q]);
                 if (c == j) l[q] = -t;
                 e[q] = t;
-                if (r == j + 1 && r < P) publish(r, t);
+                if (r == j + 2) S.R[j & 1][c] = t;   // the next step's row (the first of its warp's)
             }
         }
+    }
+    __syncthreads();
+    if (wi < 0) return;
 #pragma unroll
     for (int q = 0; q < ROWS_PER_WARP; ++q) {
-        const int r = warp + (NTHREADS / 32) * q;
-        if (r < P && c <= r && r - c <= bw) A[(int64_t)(k0 + c) * ld + (r - c)] = c == r ? e[q] : l[q];
-        B.xinv[band][(int64_t)k0 * PANEL + r * PANEL + c] = c < r ? e[q] : c == r ? 1.0 : 0.0;
+        const int r = wi + ROW_WARPS * q;
+        if (r >= PANEL) continue;
+        const double x = r < P ? S.E[r][c] : 0.0;
+        if (r < P && c <= r && r - c <= bw) A[(int64_t)(k0 + c) * ld + (r - c)] = c == r ? x : c == r - 1 ? S.sub[r] : l[q];
+        B.xinv[band][(int64_t)k0 * PANEL + r * PANEL + c] = c < r ? x : c == r ? 1.0 : 0.0;
     }
 }
 
@@ -159,17 +187,13 @@ __device__ __forceinline__ void factor_block(const Bands &B, int band, int k0, i
 __global__ void __launch_bounds__(NTHREADS) k_ldl_diag(Bands B, int k0, int *status)
 {
     if (*status) return;
-    __shared__ double W[2][PANEL];
-    __shared__ int bad;
+    __shared__ BlockShared S;
     const int bw = B.bw, band = blockIdx.x, P = min(PANEL, B.N[band] - k0);
-    const int c = threadIdx.x & 31;
-    double e[ROWS_PER_WARP];
-#pragma unroll
-    for (int q = 0; q < ROWS_PER_WARP; ++q) {
-        const int r = (threadIdx.x >> 5) + (NTHREADS / 32) * q, hi = max(r, c), lo = min(r, c);
-        e[q] = hi < P && hi - lo <= bw ? B.a[band][(int64_t)(k0 + lo) * ((int64_t)bw + 1) + (hi - lo)] : (r == c ? 1.0 : 0.0);
+    for (int t = threadIdx.x; t < PANEL * PANEL; t += NTHREADS) {
+        const int r = t >> 5, c = t & 31, hi = max(r, c), lo = min(r, c);
+        S.E[r][c] = hi < P && hi - lo <= bw ? B.a[band][(int64_t)(k0 + lo) * ((int64_t)bw + 1) + (hi - lo)] : (r == c ? 1.0 : 0.0);
     }
-    factor_block(B, band, k0, P, e, W, bad, status);
+    factor_block(B, band, k0, P, S, status);
 }
 
 // Rows below the diagonal block, SUB_ROWS per CTA, a warp per row and a lane per
@@ -214,8 +238,8 @@ __global__ void __launch_bounds__(NTHREADS) k_ldl_subpanel(Bands B, int k0, cons
 // next panel's diagonal block, goes on to factor it while the others update theirs.
 // FP64-bound where there are tiles enough: at a half bandwidth of 2,567 it runs at
 // the FP64 rate (105 M multiply-adds in 175 us); at 551 and two bands 342 tiles
-// leave two to three per SM: 32.7 us with the factored block, 44.8 us and
-// 24.4 us as two launches.
+// leave two to three per SM: 32.6 us with the factored block, 44.8 us and
+// 24.4 us as two launches; with few tiles the factored block bounds it: 28.3 us.
 __global__ void __launch_bounds__(NTHREADS) k_ldl_trailing(Bands B, int nb, int k0, int next, int *status)
 {
     if (*status) return;
@@ -228,9 +252,7 @@ __global__ void __launch_bounds__(NTHREADS) k_ldl_trailing(Bands B, int nb, int 
     const int tc = tile - ti * (ti + 1) / 2;
     __shared__ double Li[PANEL][32];       // L(i, p) * d_p, [p][a]
     __shared__ double Lc[32][PANEL + 1];   // L(c, p), [b][p]
-    __shared__ double E[PANEL][PANEL + 1]; // the next diagonal block
-    __shared__ double W[2][PANEL];
-    __shared__ int bad;
+    __shared__ BlockShared S;              // the next diagonal block
     double *A = B.a[band];
     const int64_t ld = (int64_t)bw + 1;
     const int P = min(PANEL, B.N[band] - k0), k1 = k0 + P;
@@ -265,26 +287,23 @@ __global__ void __launch_bounds__(NTHREADS) k_ldl_trailing(Bands B, int nb, int 
             old[h] = in ? A[(int64_t)(k1 + cc[h]) * ld + (r - cc[h])] : 0.0;
             sum[h] = 0.0;
         }
-        for (int t = threadIdx.x; t < PANEL * PANEL; t += NTHREADS) E[t >> 5][t & 31] = (t >> 5) == (t & 31) ? 1.0 : 0.0;
+        for (int t = threadIdx.x; t < PANEL * PANEL; t += NTHREADS) S.E[t >> 5][t & 31] = (t >> 5) == (t & 31) ? 1.0 : 0.0;
         __syncthreads();
 #pragma unroll
         for (int h = 0; h < 3; ++h)
             if (rr[h] >= 0) {
 #pragma unroll 8
                 for (int p = 0; p < PANEL; ++p) sum[h] = fma(Li[p][rr[h]], Lc[cc[h]][p], sum[h]);
-                E[rr[h]][cc[h]] = E[cc[h]][rr[h]] = old[h] - sum[h];
+                S.E[rr[h]][cc[h]] = S.E[cc[h]][rr[h]] = old[h] - sum[h];
             }
-        __syncthreads();
-        double row[ROWS_PER_WARP];
-#pragma unroll
-        for (int q = 0; q < ROWS_PER_WARP; ++q) row[q] = E[b0 + 8 * q][a];
-        factor_block(B, band, k1, Pn, row, W, bad, status);
+        factor_block(B, band, k1, Pn, S, status);
         return;
     }
-    double s[ROWS_PER_WARP], v[ROWS_PER_WARP];
-    bool on[ROWS_PER_WARP];
+    constexpr int COLS = PANEL / (NTHREADS / 32);   // columns of a warp
+    double s[COLS], v[COLS];
+    bool on[COLS];
 #pragma unroll
-    for (int q = 0; q < ROWS_PER_WARP; ++q) {
+    for (int q = 0; q < COLS; ++q) {
         const int c = c0 + b0 + 8 * q;
         on[q] = c < e && i >= c && i < e && i - c <= bw;
         v[q] = on[q] ? A[(int64_t)c * ld + (i - c)] : 0.0;
@@ -295,10 +314,10 @@ __global__ void __launch_bounds__(NTHREADS) k_ldl_trailing(Bands B, int nb, int 
     for (int p = 0; p < PANEL; ++p) {
         const double li = Li[p][a];
 #pragma unroll
-        for (int q = 0; q < ROWS_PER_WARP; ++q) s[q] = fma(li, Lc[b0 + 8 * q][p], s[q]);
+        for (int q = 0; q < COLS; ++q) s[q] = fma(li, Lc[b0 + 8 * q][p], s[q]);
     }
 #pragma unroll
-    for (int q = 0; q < ROWS_PER_WARP; ++q) {
+    for (int q = 0; q < COLS; ++q) {
         const int c = c0 + b0 + 8 * q;
         if (on[q]) A[(int64_t)c * ld + (i - c)] = v[q] - s[q];
     }
