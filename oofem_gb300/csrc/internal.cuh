@@ -201,6 +201,7 @@ struct SellMat {
     DBuf<int> sl_width;     // blocks per row of each slice
     int max_width = 0;
     DBuf<int> col;          // nslots
+    DBuf<int> slot_blk;     // node block of each slot (-1: padding); matrices of a model
     DBuf<int64_t> diag;     // slot of the diagonal block of each row (nslices*32)
     DBuf<double> v64;       // nslots * ND*ND
     DBuf<float> v32;
@@ -379,7 +380,6 @@ struct ogb_model {
     ogb::DBuf<int64_t> node_rowbase;   // CSR position of the first row of each node
     ogb::DBuf<int> node_rowlen;
     ogb::DBuf<int> act;                // active-node index per node (-1: all DOFs prescribed)
-    ogb::DBuf<int64_t> blk_slot;       // SELL slot per node block (-1: none)
     // element buffers
     ogb::DBuf<double> ke;       // nelem x nnpe x nnpe x ndofpn x ndofpn
     ogb::DBuf<double> fe;       // nelem x nnpe x ndofpn

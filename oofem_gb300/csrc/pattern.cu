@@ -621,7 +621,7 @@ __global__ void k_slice_width(int nslices, const int *width, int *sl_width, int6
 template <int ND>
 __global__ void k_fill_sell(int nrows_pad, int nact, const int *rownode, const int64_t *nb_ptr, const int *nb_col,
                             const int *act, const int64_t *sl_ptr, const int *sl_width, int *col, int64_t *diag,
-                            int64_t *blk_slot, double *v64, float *v32)
+                            int *slot_blk, double *v64, float *v32)
 {
     int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= nrows_pad) return;
@@ -634,13 +634,10 @@ __global__ void k_fill_sell(int nrows_pad, int nact, const int *rownode, const i
         for (int64_t k = nb_ptr[A]; k < nb_ptr[A + 1]; ++k) {
             int B = nb_col[k];
             int b = act[B];
-            if (b < 0) {
-                blk_slot[k] = -1;
-                continue;
-            }
+            if (b < 0) continue;
             int64_t slot = base + (int64_t)kk * 32 + r;
             col[slot] = b;
-            blk_slot[k] = slot;
+            slot_blk[slot] = (int)k;
             if (B == A) diag[a] = slot;
             ++kk;
         }
@@ -754,17 +751,18 @@ int build_sell(ogb_model *md, ogb_mtrx *m)
     OGB_CHECK(S.diag.alloc(nrows_pad));
     OGB_CHECK(S.v64.alloc((size_t)nslots * nd * nd));
     OGB_CHECK(S.v32.alloc((size_t)nslots * nd * nd));
-    OGB_CHECK(md->blk_slot.alloc(md->nblocks > 0 ? md->nblocks : 1));
+    OGB_CHECK(S.slot_blk.alloc(nslots));
+    OGB_CUDA(cudaMemsetAsync(S.slot_blk.p, 0xff, (size_t)nslots * sizeof(int), st));   // -1: padding
     OGB_CUDA(cudaMemsetAsync(S.v64.p, 0, (size_t)nslots * nd * nd * sizeof(double), st));
     OGB_CUDA(cudaMemsetAsync(S.v32.p, 0, (size_t)nslots * nd * nd * sizeof(float), st));
     if (nd == 3)
         k_fill_sell<3><<<nblk(nrows_pad), NTHREADS, 0, st>>>(nrows_pad, S.nact, rownode.p, md->nb_ptr.p, md->nb_col.p,
                                                              md->act.p, S.sl_ptr.p, S.sl_width.p, S.col.p, S.diag.p,
-                                                             md->blk_slot.p, S.v64.p, S.v32.p);
+                                                             S.slot_blk.p, S.v64.p, S.v32.p);
     else
         k_fill_sell<2><<<nblk(nrows_pad), NTHREADS, 0, st>>>(nrows_pad, S.nact, rownode.p, md->nb_ptr.p, md->nb_col.p,
                                                              md->act.p, S.sl_ptr.p, S.sl_width.p, S.col.p, S.diag.p,
-                                                             md->blk_slot.p, S.v64.p, S.v32.p);
+                                                             S.slot_blk.p, S.v64.p, S.v32.p);
     OGB_CHECK(S.ns_of_eq.alloc(md->neq > 0 ? md->neq : 1));
     k_ns_of_eq<<<nblk(nn), NTHREADS, 0, st>>>(nn, nd, md->eq.p, md->act.p, S.ns_of_eq.p);
     count_launch(ctx, 2);

@@ -579,3 +579,38 @@ def test_coarse_preconditioner(mesh, size, native_lib):
     assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]
     assert out[0][1] < out[2][1], (out[0][1], out[2][1])
     print(mesh, size, "iterations", out[0][1], "without", out[2][1])
+
+
+@pytest.mark.parametrize("mesh,size", [("hex", (1, 1, 1)), ("hex", (3, 2, 1)), ("hex", (33, 5, 4)), ("quad", 3), ("quad", 32),
+                                       ("quad", 45), ("tet", 2), ("tet", 9)])
+def test_gather_with_scattered_supports(mesh, size, ctx, native_lib, oracle):
+    """Assembly into the CSR values and the node-block copy together, at sizes around
+    a slice (32 rows) with supports scattered over single DOFs and whole nodes: the
+    CSR values against the oracle's serial sums (1e-12 of the largest), and the copy
+    through FP64 and mixed solves (1e-13 and 1e-10) against a direct solve of the
+    oracle's matrix, to the tolerances times a condition number below 1e5."""
+    import scipy.sparse as sp
+    import scipy.sparse.linalg as sl
+    from oofem_gb300 import meshgen as mg
+    m = mg.hex_cantilever(*size, jitter=0.2, seed=3) if mesh == "hex" else \
+        mg.quad_rve(size, seed=3) if mesh == "quad" else mg.tet_cube_linear(size, jitter=0.15, seed=3)
+    rng = np.random.default_rng(8)
+    m.bc_mask[rng.random(m.bc_mask.shape) < 0.15] = 1
+    m.bc_mask[rng.random(len(m.bc_mask)) < 0.1] = 1
+    m.nodal_load[:] = rng.uniform(-1.0, 1.0, m.nodal_load.shape) * (m.bc_mask == 0)
+    m.bc_value[:] = 0.0
+    model = native_lib.GpuModel(ctx, m)
+    A = native_lib.GpuCsrMtrx(ctx)
+    u, _, info = model.linear_static(A, rtol=1e-13, maxit=100000)
+    assert info.status == 0
+    neq, _, eq = oracle.number_equations(m.bc_mask)
+    rp, ci = A.pattern()
+    K = oracle.assemble_tangent(oracle.mesh_dict(m), oracle.location_arrays(m.conn, eq), neq, rp, ci, None)
+    assert rel(A.values(), K) < 1e-12
+    f = np.zeros(neq)
+    eq = np.asarray(eq).reshape(m.bc_mask.shape)
+    f[eq[eq > 0] - 1] = m.nodal_load[eq > 0]
+    x = sl.spsolve(sp.csr_matrix((K, ci, rp), shape=(neq, neq)).tocsc(), f)
+    assert rel(u.reshape(eq.shape)[eq > 0], x[eq[eq > 0] - 1]) < 1e-8
+    v, _, info = model.linear_static(A, rtol=1e-10, maxit=100000, precision=native_lib.PREC_MIXED)
+    assert info.status == 0 and rel(v.reshape(eq.shape)[eq > 0], x[eq[eq > 0] - 1]) < 1e-5
