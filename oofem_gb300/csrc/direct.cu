@@ -104,12 +104,13 @@ __global__ void k_ldl_fill(int n, int mid, const int64_t *__restrict__ rowptr, c
 // rows are held by the six warps of the other three partitions. One barrier per step.
 // (Three barriers and a division in every row: 52 us per block; rows in eight warps,
 // the reciprocal taken by the next row's owner among its other updates: 24.8 us; this:
-// 22.4 us. A dependent FP64 division takes 364 cycles, 688 beside a second warp.) A zero
-// or non-finite pivot sets *status to the 1-based equation of the band (negative: second
-// band) and stops every later launch.
+// 17.8 us; with l stored negated, an FP64 addition per row and step, 22.4 us. A dependent
+// FP64 division takes 364 cycles, 688 beside a second warp.) A zero or non-finite pivot
+// sets *status to the 1-based equation of the band (negative: second band) and stops every
+// later launch.
 constexpr int PIVOT = 3, ROW_WARPS = 6, ROWS_PER_WARP = (PANEL + ROW_WARPS - 1) / ROW_WARPS;
 struct BlockShared {
-    double E[PANEL][PANEL + 1], W[2][PANEL], R[2][PANEL], sub[PANEL];   // R: the row handed over; sub: L(r, r - 1)
+    double E[PANEL][PANEL + 1], W[2][PANEL], R[2][PANEL], sub[PANEL];   // R: the row handed over; sub: -L(r, r - 1)
     int bad;
 };
 
@@ -154,7 +155,7 @@ __device__ __forceinline__ void factor_block(const Bands &B, int band, int k0, i
                 const double row = S.R[(j + 1) & 1][c];
                 const double f = __shfl_sync(0xffffffffu, row, j);
                 const double t = fma(-f, own, c == j ? 0.0 : row);
-                if (c == j) S.sub[j + 1] = -t;
+                if (c == j) S.sub[j + 1] = t;
                 own = pivot(j + 1, t);
             }
         } else if (wi >= 0) {
@@ -165,7 +166,7 @@ __device__ __forceinline__ void factor_block(const Bands &B, int band, int k0, i
                 if (r <= j + 1 || r >= P) continue;
                 const double f = __shfl_sync(0xffffffffu, e[q], j);
                 const double t = fma(-f, w, c == j ? 0.0 : e[q]);
-                if (c == j) l[q] = -t;
+                if (c == j) l[q] = t;
                 e[q] = t;
                 if (r == j + 2) S.R[j & 1][c] = t;   // the next step's row (the first of its warp's)
             }
@@ -178,7 +179,7 @@ __device__ __forceinline__ void factor_block(const Bands &B, int band, int k0, i
         const int r = wi + ROW_WARPS * q;
         if (r >= PANEL) continue;
         const double x = r < P ? S.E[r][c] : 0.0;
-        if (r < P && c <= r && r - c <= bw) A[(int64_t)(k0 + c) * ld + (r - c)] = c == r ? x : c == r - 1 ? S.sub[r] : l[q];
+        if (r < P && c <= r && r - c <= bw) A[(int64_t)(k0 + c) * ld + (r - c)] = c == r ? x : c == r - 1 ? -S.sub[r] : -l[q];
         B.xinv[band][(int64_t)k0 * PANEL + r * PANEL + c] = c < r ? x : c == r ? 1.0 : 0.0;
     }
 }
@@ -238,8 +239,8 @@ __global__ void __launch_bounds__(NTHREADS) k_ldl_subpanel(Bands B, int k0, cons
 // next panel's diagonal block, goes on to factor it while the others update theirs.
 // FP64-bound where there are tiles enough: at a half bandwidth of 2,567 it runs at
 // the FP64 rate (105 M multiply-adds in 175 us); at 551 and two bands 342 tiles
-// leave two to three per SM: 32.6 us with the factored block, 44.8 us and
-// 24.4 us as two launches; with few tiles the factored block bounds it: 28.3 us.
+// leave two to three per SM: 32.4 us with the factored block, 44.8 us and
+// 24.4 us as two launches; with few tiles the factored block bounds it: 23.7 us.
 __global__ void __launch_bounds__(NTHREADS) k_ldl_trailing(Bands B, int nb, int k0, int next, int *status)
 {
     if (*status) return;
