@@ -231,26 +231,70 @@ __global__ void __launch_bounds__(NTHREADS) k_ldl_subpanel(Bands B, int k0, cons
 
 // Trailing update of panel [k0, k1) on the band rows/columns [k1, e),
 // e = min(N, k1 + bw): A(i, c) -= sum_p L(i, p) d_p L(c, p) for c <= i, both
-// within the band of the panel column p. One CTA per 32 x 32 tile of the lower
-// triangle; the panel rows of the tile are staged in shared memory (Li transposed,
-// so the lanes read consecutive words). Lane a takes row i0 + a, so the lanes of
-// a warp read and write 32 consecutive entries of one band column; the four columns
-// of a warp are four independent chains. With `next`, the CTA of tile (0, 0), the
-// next panel's diagonal block, goes on to factor it while the others update theirs.
-// FP64-bound where there are tiles enough: at a half bandwidth of 2,567 it runs at
-// the FP64 rate (105 M multiply-adds in 175 us); at 551 and two bands 342 tiles
-// leave two to three per SM: 32.4 us with the factored block, 44.8 us and
-// 24.4 us as two launches; with few tiles the factored block bounds it: 23.7 us.
-__global__ void __launch_bounds__(NTHREADS) k_ldl_trailing(Bands B, int nb, int k0, int next, int *status)
+// within the band of the panel column p. With `next` the first CTA of each band updates
+// the next panel's diagonal block and goes on to factor it. The other CTAs' warps share
+// the rest by items of 32 rows (a lane each) and one column, row tile by row tile: a warp
+// keeps its tile's panel rows in registers, lane p holds d_p L(c, p), handed to all lanes
+// in turn, and the next item is loaded during the 32 multiply-adds of this one. FP64-bound:
+// equal runs of items give every SM the same share to within one item per warp, where
+// 32 x 32 tiles went over the SMs in whole rounds (half bandwidth 551 and two bands, 342
+// tiles: three rounds, 32.4 us; items: 24.8 us, the factored block 23 of it).
+__device__ __forceinline__ void update_items(const Bands &B, int band, int k0, int lo, int hi)
 {
-    if (*status) return;
-    // both bands' first tiles come first: they factor the next diagonal blocks
-    const int band = blockIdx.x % nb, tile = blockIdx.x / nb, bw = B.bw;
-    // tile of the lower triangle: row ti has ti + 1 tiles
+    if (lo >= hi) return;
+    const int bw = B.bw, lane = threadIdx.x & 31, j = k0 + lane;
+    double *A = B.a[band];
+    const int64_t ld = (int64_t)bw + 1;
+    const int P = min(PANEL, B.N[band] - k0), k1 = k0 + P;
+    const int e = (int)min((int64_t)B.N[band], (int64_t)k1 + bw);
+    const double d = lane < P ? A[(int64_t)j * ld] : 0.0;
+    // row tile ti holds the items [base, base + 32 (ti + 1)): columns k1, k1 + 1, ...
+    const int tile = lo >> 5;
     int ti = (int)((sqrtf(8.0f * tile + 1.0f) - 1.0f) * 0.5f);
     while ((ti + 1) * (ti + 2) / 2 <= tile) ++ti;
     while (ti * (ti + 1) / 2 > tile) --ti;
-    const int tc = tile - ti * (ti + 1) / 2;
+    int base = 16 * ti * (ti + 1);
+    auto load = [&](int row, int c, double &l, double &v) {
+        l = lane < P && c < e && c - j <= bw ? A[(int64_t)j * ld + (c - j)] : 0.0;
+        v = c < e && row >= c && row < e && row - c <= bw ? A[(int64_t)c * ld + (row - c)] : 0.0;
+    };
+    double l, v;
+    load(k1 + 32 * ti + lane, k1 + lo - base, l, v);
+    for (int it = lo; it < hi; ++ti, base = 16 * ti * (ti + 1)) {
+        const int row = k1 + 32 * ti + lane, end = min(hi, base + 32 * (ti + 1));
+        double li[PANEL];
+#pragma unroll
+        for (int p = 0; p < PANEL; ++p)
+            li[p] = p < P && row < e && row - (k0 + p) <= bw ? A[(int64_t)(k0 + p) * ld + (row - (k0 + p))] : 0.0;
+#pragma unroll 1
+        for (; it < end; ++it) {
+            const int c = k1 + it - base;
+            const double lc = l * d, old = v;
+            if (it + 1 < hi) {
+                const bool same = it + 1 < base + 32 * (ti + 1);
+                load(same ? row : row + 32, same ? c + 1 : k1, l, v);
+            }
+            double sum = 0.0;
+#pragma unroll
+            for (int p = 0; p < PANEL; ++p) sum = fma(li[p], __shfl_sync(0xffffffffu, lc, p), sum);
+            if (c < e && row >= c && row < e && row - c <= bw) A[(int64_t)c * ld + (row - c)] = old - sum;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(NTHREADS) k_ldl_trailing(Bands B, int nb, int k0, int nt, int next, int *status)
+{
+    if (*status) return;
+    // the bands alternate over the CTAs; with `next` each band's first CTA factors
+    const int band = blockIdx.x % nb, cta = blockIdx.x / nb - (next ? 1 : 0);
+    if (cta >= 0) {
+        constexpr int W = NTHREADS / 32;
+        const int first = next ? 32 : 0, items = 16 * nt * (nt + 1) - first;
+        const int64_t warps = (int64_t)(gridDim.x / nb - (next ? 1 : 0)) * W, w = (int64_t)cta * W + (threadIdx.x >> 5);
+        update_items(B, band, k0, first + (int)(items * w / warps), first + (int)(items * (w + 1) / warps));
+        return;
+    }
+    const int bw = B.bw;
     __shared__ double Li[PANEL][32];       // L(i, p) * d_p, [p][a]
     __shared__ double Lc[32][PANEL + 1];   // L(c, p), [b][p]
     __shared__ BlockShared S;              // the next diagonal block
@@ -258,70 +302,43 @@ __global__ void __launch_bounds__(NTHREADS) k_ldl_trailing(Bands B, int nb, int 
     const int64_t ld = (int64_t)bw + 1;
     const int P = min(PANEL, B.N[band] - k0), k1 = k0 + P;
     const int e = (int)min((int64_t)B.N[band], (int64_t)k1 + bw);
-    const int i0 = k1 + 32 * ti, c0 = k1 + 32 * tc;
-    const bool diag = next && tile == 0;
     const int a = threadIdx.x & 31, b0 = threadIdx.x >> 5;
-    const int i = i0 + a;
+    const int i = k1 + a;
 #pragma unroll
     for (int q = 0; q < PANEL / (NTHREADS / 32); ++q) {
-        const int p = b0 + q * (NTHREADS / 32), j = k0 + p, c = c0 + a;
+        const int p = b0 + q * (NTHREADS / 32), j = k0 + p, c = k1 + a;
         const double *cjp = A + (int64_t)j * ld;
         Li[p][a] = (p < P && i < e && i - j <= bw) ? cjp[i - j] * cjp[0] : 0.0;
         Lc[a][p] = (p < P && c < e && c - j <= bw) ? cjp[c - j] : 0.0;
     }
-    if (diag) {
-        // lower triangle of the next diagonal block, 528 entries packed over the
-        // threads (half the FP64 work of the tile), handed over through shared memory
-        const int Pn = min(PANEL, B.N[band] - k1);
-        double old[3], sum[3];
-        int rr[3], cc[3];
+    // lower triangle of the next diagonal block, 528 entries packed over the
+    // threads (half the FP64 work of the tile), handed over through shared memory
+    const int Pn = min(PANEL, B.N[band] - k1);
+    double old[3], sum[3];
+    int rr[3], cc[3];
 #pragma unroll
-        for (int h = 0; h < 3; ++h) {
-            const int t = threadIdx.x + h * NTHREADS;
-            int r = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
-            if ((r + 1) * (r + 2) / 2 <= t) ++r;
-            if (r * (r + 1) / 2 > t) --r;
-            rr[h] = r;
-            cc[h] = t - r * (r + 1) / 2;
-            const bool in = t < PANEL * (PANEL + 1) / 2 && r < Pn && r - cc[h] <= bw;
-            if (!in) rr[h] = -1;
-            old[h] = in ? A[(int64_t)(k1 + cc[h]) * ld + (r - cc[h])] : 0.0;
-            sum[h] = 0.0;
-        }
-        for (int t = threadIdx.x; t < PANEL * PANEL; t += NTHREADS) S.E[t >> 5][t & 31] = (t >> 5) == (t & 31) ? 1.0 : 0.0;
-        __syncthreads();
-#pragma unroll
-        for (int h = 0; h < 3; ++h)
-            if (rr[h] >= 0) {
-#pragma unroll 8
-                for (int p = 0; p < PANEL; ++p) sum[h] = fma(Li[p][rr[h]], Lc[cc[h]][p], sum[h]);
-                S.E[rr[h]][cc[h]] = S.E[cc[h]][rr[h]] = old[h] - sum[h];
-            }
-        factor_block(B, band, k1, Pn, S, status);
-        return;
+    for (int h = 0; h < 3; ++h) {
+        const int t = threadIdx.x + h * NTHREADS;
+        int r = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
+        if ((r + 1) * (r + 2) / 2 <= t) ++r;
+        if (r * (r + 1) / 2 > t) --r;
+        rr[h] = r;
+        cc[h] = t - r * (r + 1) / 2;
+        const bool in = t < PANEL * (PANEL + 1) / 2 && r < Pn && r - cc[h] <= bw;
+        if (!in) rr[h] = -1;
+        old[h] = in ? A[(int64_t)(k1 + cc[h]) * ld + (r - cc[h])] : 0.0;
+        sum[h] = 0.0;
     }
-    constexpr int COLS = PANEL / (NTHREADS / 32);   // columns of a warp
-    double s[COLS], v[COLS];
-    bool on[COLS];
-#pragma unroll
-    for (int q = 0; q < COLS; ++q) {
-        const int c = c0 + b0 + 8 * q;
-        on[q] = c < e && i >= c && i < e && i - c <= bw;
-        v[q] = on[q] ? A[(int64_t)c * ld + (i - c)] : 0.0;
-        s[q] = 0.0;
-    }
+    for (int t = threadIdx.x; t < PANEL * PANEL; t += NTHREADS) S.E[t >> 5][t & 31] = (t >> 5) == (t & 31) ? 1.0 : 0.0;
     __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 3; ++h)
+        if (rr[h] >= 0) {
 #pragma unroll 8
-    for (int p = 0; p < PANEL; ++p) {
-        const double li = Li[p][a];
-#pragma unroll
-        for (int q = 0; q < COLS; ++q) s[q] = fma(li, Lc[b0 + 8 * q][p], s[q]);
-    }
-#pragma unroll
-    for (int q = 0; q < COLS; ++q) {
-        const int c = c0 + b0 + 8 * q;
-        if (on[q]) A[(int64_t)c * ld + (i - c)] = v[q] - s[q];
-    }
+            for (int p = 0; p < PANEL; ++p) sum[h] = fma(Li[p][rr[h]], Lc[cc[h]][p], sum[h]);
+            S.E[rr[h]][cc[h]] = S.E[cc[h]][rr[h]] = old[h] - sum[h];
+        }
+    factor_block(B, band, k1, Pn, S, status);
 }
 
 // The second band's updates of the middle rows are added to the first band's
@@ -830,12 +847,15 @@ static int ldl_factor_in(ogb_mtrx *m, bool natural, int *pivot)
             }
             k_ldl_subpanel<<<dim3((unsigned)ceil_div(e - k1, SUB_ROWS), nb), NTHREADS, 0, s>>>(B, k0, st);
             const unsigned nt = (unsigned)ceil_div(e - k1, 32);
-            // few tiles: one CTA per SM (by its shared memory), so that no tile shares
-            // the FP64 pipe of the CTA that factors the next block, the longest of
-            // the launch (60 x 12 x 12 hexes: 32.7 us against 44.8 us); from four per SM on the
-            // tiles take longer than that block, and several per SM hide their loads
-            const size_t excl = (int64_t)(nt * (nt + 1) / 2) * nb <= 4 * (int64_t)num_sms() ? EXCLUSIVE_SMEM : 0;
-            k_ldl_trailing<<<nt * (nt + 1) / 2 * nb, NTHREADS, excl, s>>>(B, nb, k0, k1 < kb1 ? 1 : 0, st);
+            // few items: one CTA per SM (by its shared memory), so that none shares the FP64
+            // pipe of the CTA that factors the next block, the longest of the launch
+            // (60 x 12 x 12 hexes, by tiles: 32.4 us against 44.8 us); from 128 per SM on
+            // they take longer than that block, and two CTAs per SM hide their loads
+            const int64_t items = 16 * nt * ((int64_t)nt + 1) * nb;
+            const bool few = items <= 128 * (int64_t)num_sms();
+            const int next = k1 < kb1 ? 1 : 0, ctas = (few ? 1 : 2) * num_sms() / nb - next;
+            const int work = (int)std::max<int64_t>(1, std::min<int64_t>(ctas, ceil_div(items / nb, NTHREADS / 32)));
+            k_ldl_trailing<<<(work + next) * nb, NTHREADS, few ? EXCLUSIVE_SMEM : 0, s>>>(B, nb, k0, (int)nt, next, st);
             count_launch(ctx, 2);
         }
     };

@@ -243,3 +243,19 @@ def test_direct_zero_pivot_of_the_far_end(native_lib):
     assert K[n - 1, n - 1] == 0.0
     b = np.random.default_rng(1).standard_normal(n)
     assert rel(A.ldlt_solve(b), np.linalg.solve(K, b)) < 1e-10
+
+
+@pytest.mark.parametrize("n", [40, 97, 700, 3000])
+def test_direct_wide_bands(n, native_lib):
+    """Random graphs, whose band stays wide in any order: few to many row tiles below a
+    panel (the rank-32 update's items fewer than the warps, several per warp across row
+    tiles, and two CTAs per SM), against numpy. The eigenvalues lie between 1 and 100 (at
+    most a few dozen edges at a node): 1e-12 suffices for a factorization's rounding."""
+    rng = np.random.default_rng(n)
+    pairs = rng.integers(0, n, (4 * n, 2))
+    pairs = np.unique(np.sort(pairs[pairs[:, 0] != pairs[:, 1]], axis=1), axis=0)
+    locs = [np.array([i + 1]) for i in range(n)] + [p + 1 for p in pairs]
+    kes = [np.array([[1.0]])] * n + [w * np.array([[1.0, -1.0], [-1.0, 1.0]]) for w in rng.uniform(0.1, 1.5, len(pairs))]
+    A, K = assembled(native_lib, n, locs, kes)
+    b = rng.standard_normal(n)
+    assert rel(A.ldlt_solve(b), np.linalg.solve(K, b)) < 1e-12
